@@ -1335,7 +1335,7 @@ DEV void scal_stats(SolveState* G, const Solve<T>& K, int second, double true_re
 // mode 8/9: same matrix and hierarchy, density correction counted as solved).
 template <class M>
 __global__ void __launch_bounds__(NT, 2) k_mgpcg(DevScene d, int second, int scale_mode) {
-    grid_begin();
+    grid_begin(d.K);
     using acc = typename M::acc;
     using acc4 = typename M::acc4;
     __shared__ TileCache tc;
@@ -1549,7 +1549,7 @@ size_t pressure_batch_smem(const Levels& lv) {
 
 template <class M>
 __global__ void __launch_bounds__(NT, 4) k_mgpcg_batch(BatchView B, int second) {
-    grid_begin();
+    grid_begin(B.K);
     using acc = typename M::acc;
     using acc4 = typename M::acc4;
     __shared__ TileCache tc;

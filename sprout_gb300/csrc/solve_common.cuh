@@ -54,15 +54,35 @@ DEV unsigned long long global_ns() {
     return t;
 }
 
-// The number of grid barriers this block has passed in the current launch (one per block, in
-// shared memory; grid_begin sets it to zero at the start of every persistent kernel).
-DEV uint32_t& grid_epoch() {
-    __shared__ uint32_t epoch;
-    return epoch;
+// What a block keeps of a launch's grid barriers in shared memory: how many it has passed, and
+// the settings of SolveState that do not change during a launch (read once, in grid_begin: a
+// barrier that read them before its arrival would wait for global memory each time).
+struct GridState {
+    uint32_t epoch, spin_limit, stall_ns, dbg_block;
+    unsigned long long* trace;
+    uint32_t trace_rows, trace_cols, trace_base;
+    int ok;
+};
+DEV GridState& grid_state() {
+    __shared__ GridState g;
+    return g;
 }
-DEV void grid_begin() {
-    if (threadIdx.x == 0) grid_epoch() = 0u;
+DEV void grid_begin(const SolveState* K) {
+    if (threadIdx.x == 0)
+        grid_state() = GridState{0u, K->dbg_spin_limit != 0u ? K->dbg_spin_limit : SPIN_LIMIT, K->dbg_stall_ns, K->dbg_block,
+                                 K->trace, K->trace_rows, K->trace_cols, K->trace_base, K->error == 0u ? 1 : 0};
     __syncthreads();
+}
+// the barrier's rare parts: failure injection (tests only, off unless set: this block arrives
+// late, by a wait bounded by the device clock, at most a second, and by a poll count) ...
+static __device__ __noinline__ void grid_stall(uint32_t stall) {
+    const unsigned long long t0 = global_ns();
+    const unsigned long long lim = stall < 1000000000u ? stall : 1000000000u;
+    for (uint32_t k = 0; k < (1u << 21) && global_ns() - t0 < lim; k++) __nanosleep(500);
+}
+// ... and the phase trace's row of the barrier a block has come to
+static __device__ __noinline__ void grid_trace(const GridState& G, int col) {
+    if (blockIdx.x + 1 < G.trace_cols) G.trace[(size_t)((G.trace_base + G.epoch) % G.trace_rows) * G.trace_cols + col] = global_ns();
 }
 
 // Grid-wide barrier over the co-resident blocks of a cooperative launch: one arrival counter
@@ -71,63 +91,50 @@ DEV void grid_begin() {
 // (bounded spin) until the counter reaches (e + 1) x blocks, which the last block to arrive
 // makes true with its own add: releasing costs no store beyond the arrivals, and no block
 // waits for its arrival's round trip before it starts to poll. Returns false (and every
-// block leaves) once any wait has run out.
+// block leaves) once any wait has run out: a block that finds its own wait over goes on to the
+// next barrier, where the blocks that left are missing, and leaves there. A launch that starts
+// with the error word set does nothing.
+//
+// Nothing is read from global memory before the arrival: the error word, the injection's and
+// the trace's settings read there cost two to three trips to L2 (~0.8 us) per barrier, of which
+// a pressure iteration has 5 to 13. Reading them once per launch took a 384 x 216 dam break from
+// 0.64 to 0.61 ms a substep and a solve of 128 x 72 from 570 to 537 us.
 DEV bool grid_sync(SolveState* K) {
-    __shared__ int s_ok;
+    GridState& G = grid_state();
+    if (!G.ok) return false;
     __syncthreads();
     if (threadIdx.x == 0) {
         int ok = 1;
-        volatile uint32_t* vcnt = &K->bar_count;
         volatile uint32_t* verr = &K->error;
-        unsigned long long* trace = K->trace;
-        const uint32_t epoch = grid_epoch();
-        grid_epoch() = epoch + 1u;
-        if (*verr != 0u) {
-            ok = 0;
-        } else {
-            // failure injection (tests only, off unless set): this block arrives late, by a
-            // wait bounded by the device clock (at most a second) and by a poll count
-            const uint32_t stall = K->dbg_stall_ns;
-            if (stall != 0u && blockIdx.x == K->dbg_block) {
-                const unsigned long long t0 = global_ns();
-                const unsigned long long lim = stall < 1000000000u ? stall : 1000000000u;
-                for (uint32_t k = 0; k < (1u << 21) && global_ns() - t0 < lim; k++) __nanosleep(500);
-            }
-            const uint32_t spin_limit = K->dbg_spin_limit != 0u ? K->dbg_spin_limit : SPIN_LIMIT;
-            const unsigned long long t_in = trace ? global_ns() : 0ull;
-            const uint32_t base = trace ? *(volatile uint32_t*)&K->trace_base : 0u;
-            // the arrival releases the block's writes (ordered before it by the block barrier
-            // above; release is cumulative), the acquiring reads of the wait make the other
-            // blocks' writes visible to this block after the block barrier below; this
-            // thread's own add is ordered before its later loads of the same word
-            asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&K->bar_count) : "memory");
-            const uint32_t target = (epoch + 1u) * gridDim.x;
-            unsigned long long* row = nullptr;
-            if (trace && blockIdx.x + 1 < K->trace_cols) {
-                row = trace + (size_t)((base + epoch) % K->trace_rows) * K->trace_cols;
-                row[blockIdx.x] = t_in;
-            }
-            uint32_t spins = 0;
-            for (;;) {
-                uint32_t now;
-                asm volatile("ld.acquire.gpu.u32 %0, [%1];" : "=r"(now) : "l"(&K->bar_count) : "memory");
-                if (now >= target) break;
-                if (*verr != 0u) { ok = 0; break; }
-                if (++spins > spin_limit) {
-                    if (atomicOr(&K->error, ERR_TIMEOUT) == 0u) {
-                        K->err_arrived = *vcnt - epoch * gridDim.x;
-                        K->err_blocks = gridDim.x;
-                    }
-                    ok = 0;
-                    break;
+        if (G.stall_ns != 0u && blockIdx.x == G.dbg_block) grid_stall(G.stall_ns);
+        if (G.trace) grid_trace(G, (int)blockIdx.x);
+        // the arrival releases the block's writes (ordered before it by the block barrier
+        // above; release is cumulative), the acquiring reads of the wait make the other
+        // blocks' writes visible to this block after the block barrier below; this
+        // thread's own add is ordered before its later loads of the same word
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&K->bar_count) : "memory");
+        const uint32_t epoch = G.epoch, target = (epoch + 1u) * gridDim.x;
+        uint32_t spins = 0;
+        for (;;) {
+            uint32_t now;
+            asm volatile("ld.acquire.gpu.u32 %0, [%1];" : "=r"(now) : "l"(&K->bar_count) : "memory");
+            if (now >= target) break;
+            if ((++spins & 15u) == 0u && *verr != 0u) { ok = 0; break; }
+            if (spins > G.spin_limit) {
+                if (atomicOr(&K->error, ERR_TIMEOUT) == 0u) {
+                    K->err_arrived = *(volatile uint32_t*)&K->bar_count - epoch * gridDim.x;
+                    K->err_blocks = gridDim.x;
                 }
+                ok = 0;
+                break;
             }
-            if (row && blockIdx.x == 0) row[K->trace_cols - 1] = global_ns();
         }
-        s_ok = ok;
+        if (G.trace && blockIdx.x == 0) grid_trace(G, (int)G.trace_cols - 1);
+        G.epoch = epoch + 1u;
+        G.ok = ok;
     }
     __syncthreads();
-    return s_ok != 0;
+    return G.ok != 0;
 }
 
 // Asynchronous copies global -> shared (cp.async, N = 4, 8 or 16 bytes, both addresses

@@ -929,7 +929,7 @@ struct VSolve {
 // pressure solve changed the velocity since visc_setup).
 template <int NU>
 __global__ void __launch_bounds__(NT, 2) k_visc_solve(DevScene d, int restrain) {
-    grid_begin();
+    grid_begin(d.K);
     __shared__ VSmem<NU> sm;
     __shared__ VScal K;
     __shared__ VTileCache tc;
@@ -1137,7 +1137,7 @@ DEV void vbatch_fill_cache(const VBatchView& B, VTileCache& tc) {
 
 template <int NU>
 __global__ void __launch_bounds__(NT, 2) k_visc_batch(VBatchView B) {
-    grid_begin();
+    grid_begin(B.K);
     __shared__ VSmem<NU> sm;
     __shared__ VTileCache tc;
     __shared__ int s_run;
