@@ -86,6 +86,7 @@ struct DevScene {
     // multigrid / Krylov
     float4* mga;
     float* mgd;
+    float2* mgy;        // per level cell: the diagonal and its reciprocal (recip_row)
     float2 *mgx, *mgz, *mgr, *mgr2, *cgp, *cgp2, *cgq;
     uint32_t* ptile;
     uint32_t* plist;    // per level (at lv.toff), the tiles with pressure unknowns in order

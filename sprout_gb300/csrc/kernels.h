@@ -236,6 +236,5 @@ int pressure_blocks_max(int device, size_t smem, bool mixed);
 // Dynamic shared memory of the persistent pressure kernel: the tail levels of each block.
 size_t pressure_smem(const Levels& lv);
 // ... and of the batched one, whose staging regions share it with the tail.
-size_t pressure_batch_smem(const Levels& lv);
 
 }  // namespace sprout

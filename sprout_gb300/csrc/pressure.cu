@@ -54,12 +54,11 @@ struct Plain {
     using acc4 = float4;
     DEV static float4 A(const DevScene& d, int i) { return d.mga[i]; }
     DEV static float Dg(const DevScene& d, int i) { return d.mgd[i]; }
-    DEV static void setA(const DevScene& d, int i, float4 a, float dg) { d.mga[i] = a; d.mgd[i] = dg; }
-    DEV static void setX(const DevScene& d, int i, float2 v) { d.mgx[i] = v; }
-    DEV static float2 Z(const DevScene& d, int i) { return d.mgz[i]; }
-    DEV static void setZ(const DevScene& d, int i, float2 v) { d.mgz[i] = v; }
-    DEV static float2 R(const DevScene& d, int i) { return d.mgr[i]; }   // a coarse level's rhs
-    DEV static void setR(const DevScene& d, int i, float2 v) { d.mgr[i] = v; }
+    DEV static void setA(const DevScene& d, int i, float4 a, float dg) {
+        d.mga[i] = a;
+        d.mgd[i] = dg;
+        d.mgy[i] = make_float2(dg, recip_row(dg, a));
+    }
     DEV static acc4* part(const DevScene& d) { return d.partials; }
     DEV static acc4 zero4() { return make_float4(0.0f, 0.0f, 0.0f, 0.0f); }
     // the four products a_k b_k of a cell's partial sums, and a total as the scalars use it
@@ -67,17 +66,24 @@ struct Plain {
         return make_float4(a0 * b0, a1 * b1, a2 * b2, a3 * b3);
     }
     DEV static float4 fin(acc4 a) { return a; }
-    // the stored matrix as a tile region stages it: bytes per row of couplings, their address,
-    // the diagonal's array, and the row read from its staged slot in FP32
-    static constexpr int kABytes = 16;
-    DEV static const void* Araw(const DevScene& d, int i) { return d.mga + i; }
-    DEV static const float* Dptr(const DevScene& d) { return d.mgd; }
-    DEV static float4 Aslot(const float4& slot) { return slot; }
-    // a / D with D's staged slot (the diagonal): the shader's IEEE division; quotp is zero
-    // unless the slot is positive
-    DEV static float quot(float a, float slot) { return divz(a, slot); }
-    DEV static float2 quot(float2 a, float slot) { return divz(a, slot); }
-    DEV static float quotp(float a, float slot) { return divp(a, slot); }
+    // what the smoothers read of a row: its couplings, and the diagonal with its reciprocal (zero
+    // where the cell is no unknown)
+    using Row = float4;
+    using Diag = float2;
+    DEV static const Row* rows(const DevScene& d) { return d.mga; }
+    DEV static const Diag* diags(const DevScene& d) { return d.mgy; }
+    DEV static float4 wide(const Row& a) { return a; }
+    DEV static Diag no_diag() { return make_float2(0.0f, 0.0f); }
+    DEV static bool unk(const Diag& y) { return y.x > 0.0f; }
+    DEV static float4 pack_red(float2 r, const Diag& y) { return make_float4(r.x, r.y, y.x, y.y); }
+    DEV static void unpack_red(const float4& v, float2& r, Diag& y) {
+        r = make_float2(v.x, v.y);
+        y = make_float2(v.z, v.w);
+    }
+    template <bool SLOW>
+    DEV static float2 quot(float2 a, const Diag& y) { return make_float2(quot1<SLOW>(a.x, y), quot1<SLOW>(a.y, y)); }
+    // whether a may be divided by y's diagonal the fast way (an unknown's)
+    DEV static bool ok(float2 a, const Diag& y) { return value_ok(a.x) && value_ok(a.y) && y.y > 0.0f; }
 };
 
 // a pair of BF16 values in 32 bits (x in the low half), rounded to nearest even
@@ -124,33 +130,33 @@ struct Mixed {
     // nonlinear operator, which conjugate gradients does not tolerate (it stagnates near the
     // rounding level); the matrices are fixed during a solve, so the V-cycle built on their
     // BF16 copies stays a linear, symmetric positive definite preconditioner
-    DEV static void setX(const DevScene& d, int i, float2 v) { d.mgx[i] = v; }
-    DEV static float2 Z(const DevScene& d, int i) { return d.mgz[i]; }
-    DEV static void setZ(const DevScene& d, int i, float2 v) { d.mgz[i] = v; }
-    DEV static float2 R(const DevScene& d, int i) { return d.mgr[i]; }
-    DEV static void setR(const DevScene& d, int i, float2 v) { d.mgr[i] = v; }
     DEV static acc4* part(const DevScene& d) { return d.partials; }
     DEV static acc4 zero4() { return make_float4(0.0f, 0.0f, 0.0f, 0.0f); }
     DEV static acc4 prod4(float a0, float b0, float a1, float b1, float a2, float b2, float a3, float b3) {
         return make_float4(a0 * b0, a1 * b1, a2 * b2, a3 * b3);
     }
     DEV static Dbl4 fin(acc4 a) { return Dbl4{(double)a.x, (double)a.y, (double)a.z, (double)a.w}; }
-    static constexpr int kABytes = 8;
-    DEV static const void* Araw(const DevScene& d, int i) { return d.hga + i; }
-    // the level passes stage the inverse diagonal in the diagonal's slot (positive exactly
-    // where the diagonal is) and multiply by it instead of dividing: a V-cycle is a
-    // preconditioner here, not the reference's arithmetic, and ten IEEE divisions per black
-    // cell were most of a way down's instructions
-    DEV static const float* Dptr(const DevScene& d) { return d.hgi; }
-    DEV static float quot(float a, float slot) { return a * slot; }
-    DEV static float2 quot(float2 a, float slot) { return make_float2(a.x * slot, a.y * slot); }
-    DEV static float quotp(float a, float slot) { return slot > 0.0f ? a * slot : 0.0f; }
-    // the BF16 row copied into the first 8 bytes of the slot, widened on reading
-    DEV static float4 Aslot(const float4& slot) {
-        const uint2 u = *reinterpret_cast<const uint2*>(&slot);
+    using Row = uint2;
+    // the smoothers read the inverse diagonal (positive exactly where the diagonal is) and
+    // multiply by it instead of dividing: a V-cycle is a preconditioner here, not the
+    // reference's arithmetic
+    using Diag = float;
+    DEV static const Row* rows(const DevScene& d) { return d.hga; }
+    DEV static const Diag* diags(const DevScene& d) { return d.hgi; }
+    DEV static float4 wide(const Row& u) {
         const float2 a = unpack(u.x), b = unpack(u.y);
         return make_float4(a.x, a.y, b.x, b.y);
     }
+    DEV static Diag no_diag() { return 0.0f; }
+    DEV static bool unk(const Diag& y) { return y > 0.0f; }
+    DEV static float4 pack_red(float2 r, const Diag& y) { return make_float4(r.x, r.y, y, 0.0f); }
+    DEV static void unpack_red(const float4& v, float2& r, Diag& y) {
+        r = make_float2(v.x, v.y);
+        y = v.z;
+    }
+    template <bool SLOW>
+    DEV static float2 quot(float2 a, const Diag& y) { return make_float2(a.x * y, a.y * y); }
+    DEV static bool ok(float2, const Diag&) { return true; }
 };
 
 template <class T>
@@ -176,8 +182,8 @@ DEV bool unknown_op(const DevScene& d, const Lv& L, int x, int y) { return l_ins
 
 
 // cg_scale.comp on level-0 tile t: warm start from last substep's potential rescaled to
-// this substep. Mixed: also level 0's matrix in BF16 for the V-cycle (every cell: rhs.comp
-// rewrote them all).
+// this substep. Also level 0's diagonal with its reciprocal, or (mixed) its matrix in BF16, for
+// the V-cycle (every cell: rhs.comp rewrote them all).
 template <class M>
 DEV void cg_scale_tile(const DevScene& d, int t, int mode) {
     const Lv F = lev(d.lv, 0);
@@ -189,6 +195,8 @@ DEV void cg_scale_tile(const DevScene& d, int t, int mode) {
         int m = 0;
         for (int q = 0; q < 4; q++) m |= unknown_op(d, F, cx + NBX[q], cy + NBY[q]) ? (1 << q) : 0;
         Mixed::setA(d, i, d.mga[i], d.mgd[i], m);
+    } else {
+        d.mgy[i] = make_float2(d.mgd[i], recip_row(d.mgd[i], d.mga[i]));
     }
     if (d.ptile[F.toff + t] == 0u) return;
     if (d.mgd[i] > 0.0f) {
@@ -305,88 +313,87 @@ DEV int level_tiles(const DevScene& d, int l) {
 
 // ---- the V-cycle --------------------------------------------------------------------------
 
-// The right-hand side a way down reads: level 0's residual (FP32), fused with the update
-// r -= alpha q of cg_update.comp when q is set; or a coarse level's, through M.
-template <class M>
-struct Rsrc {
-    const float2* r;      // level-0 residual before the update (null: a coarse level)
-    const float2* q;      // A p, for the fused update (null: no update)
-    float ax, ay;
-    DEV float2 at(const DevScene& d, int i) const {
-        if (!r) return M::R(d, i);
-        float2 v = r[i];
-        if (q) {
-            float2 qq = q[i];
-            v.x = v.x - ax * qq.x;
-            v.y = v.y - ay * qq.y;
-        }
-        return v;
-    }
+// The tail levels' state in each block's shared memory (dynamic, FP32 in both precisions). A
+// level's unknowns are listed by colour, the even cells first: entry p of the list holds the
+// cell's row (couplings, zero towards cells that are no unknowns; diagonal and reciprocal), its
+// slot and its right-hand side, so that a half-sweep's thread finds all of these from its own
+// number alone; the iterates lie by slot (the cells' offsets from the first tail level, the slots
+// of mg_tail.comp), where neighbours are at fixed distances. Slots that are no unknown hold zero.
+struct TailLevel {
+    int o, n, w, h;     // its cells are slots o .. o + n - 1
+    uint32_t wm;        // division constant of the width
+    int n0, n1, pad;    // unknowns with (x + y) even (entries o ..) and odd (entries o + n0 ..)
 };
-
-// The tail levels' state in each block's shared memory (dynamic, FP32 in both precisions):
-// per tail cell the matrix row (couplings, diagonal), the iterate and the right-hand side,
-// at its offset from the first tail level (the slots of mg_tail.comp).
+constexpr int kTailLevels = 16;
+constexpr uint32_t kNoEntry = 0xffffu;
 struct Tail {
-    float4* a;    // couplings of tail cells aoff .. T - 1 (at a[s - aoff])
-    float* dg;
-    float2* x;
+    float4* a;
+    float2* dy;
+    float2* x;       // (of the first level: read by the way up above the tail)
     float2* r;
-    uint8_t* m;   // per cell: bit q set when neighbour q is an unknown, bit 4 when the cell is
-    int base, T, nf;
-    int aoff;     // 0: every level's couplings in shared memory; nf: the first tail level's read
-                  // from the level's stored matrix (a batch, whose blocks then fit four per SM)
+    TailLevel* lv;
+    uint16_t* slot;  // an entry's slot
+    uint16_t* ent;   // a slot's entry (kNoEntry: no unknown)
+    int base, T, nf, nl;
 };
 
-// The couplings of tail cell s, from shared memory or (the first level of a batch's tail)
-// from the level's stored matrix: the same values tail_setup would have copied.
-template <class M>
-DEV float4 tail_a(const DevScene& d, const Tail& tl, int s) {
-    return s < tl.aoff ? M::A(d, tl.base + s) : tl.a[s - tl.aoff];
-}
+DEV bool t_unknown(const Tail& tl, const Lv& L, int x, int y) { return l_inside(L, x, y) && tl.dy[L.off - tl.base + y * L.w + x].x > 0.0f; }
 
-DEV bool t_unknown(const Tail& tl, const Lv& L, int x, int y) { return l_inside(L, x, y) && tl.dg[L.off - tl.base + y * L.w + x] > 0.0f; }
-
-// The tail of scene d laid out in the dynamic shared memory at smem; its right-hand sides at
-// r_store if given (they are live only inside the tail phase, so a caller may keep them in
-// bytes that other phases use), else after the iterates.
-DEV Tail make_tail(const DevScene& d, unsigned char* smem, float2* r_store = nullptr, bool first_global = false) {
+// A tail of T cells, the first nf of them its first level's, in nl levels, laid out in shared
+// memory at smem; its right-hand sides, live only inside the tail phase, at r.
+DEV Tail tail_at(unsigned char* smem, float2* r, int base, int T, int nf, int nl) {
     Tail tl;
-    const Lv F = lev(d.lv, d.lv.tail), E = lev(d.lv, d.lv.n - 1);
-    tl.base = F.off;
-    tl.T = E.off + E.w * E.h - F.off;
-    tl.nf = F.w * F.h;
-    tl.aoff = first_global ? tl.nf : 0;
+    tl.base = base;
+    tl.T = T;
+    tl.nf = nf;
+    tl.nl = nl;
     tl.a = reinterpret_cast<float4*>(smem);
-    tl.x = reinterpret_cast<float2*>(tl.a + (tl.T - tl.aoff));
-    if (r_store) {
-        tl.r = r_store;
-        tl.dg = reinterpret_cast<float*>(tl.x + tl.T);
-    } else {
-        tl.r = tl.x + tl.T;
-        tl.dg = reinterpret_cast<float*>(tl.r + tl.T);
-    }
-    tl.m = reinterpret_cast<uint8_t*>(tl.dg + tl.T);
+    tl.lv = reinterpret_cast<TailLevel*>(tl.a + T);
+    tl.dy = reinterpret_cast<float2*>(tl.lv + kTailLevels);
+    tl.x = tl.dy + T;
+    tl.r = r;
+    tl.slot = reinterpret_cast<uint16_t*>(tl.x + T);
+    tl.ent = tl.slot + T;
     return tl;
 }
 
-// Cells of the tail levels, and the tail's bytes with and without its right-hand sides.
-__host__ __device__ inline int tail_cells(const Levels& lv) { return lv.off[lv.n - 1] + lv.w[lv.n - 1] * lv.h[lv.n - 1] - lv.off[lv.tail]; }
-__host__ __device__ inline size_t tail_bytes(int T, bool with_r, int aoff = 0) {
-    const size_t per = sizeof(float2) + (with_r ? sizeof(float2) : 0) + sizeof(float) + 1;
-    return ((size_t)T * per + (size_t)(T - aoff) * sizeof(float4) + 15) / 16 * 16;
+// The persistent kernels' dynamic shared memory: the level passes' exchange of cell values
+// (TileSmem), whose bytes hold the tail's right-hand sides in the tail phase (no tile is being
+// computed then), and one scene's tail.
+struct TileSmem {
+    unsigned char stage[2][17408];   // two tiles' fields, staged asynchronously (LevelStage, ApplyStage)
+    float4 red[200];         // per red slot of a way down: its right-hand side, diagonal and reciprocal
+    float2 black[200];       // per black slot: its new value
+    float2 prod[NT];         // per cell: its two products of the tile's sums
+};
+constexpr size_t kTileBytes = sizeof(TileSmem);
+static_assert(kTileBytes % 16 == 0, "the tail follows");
+static_assert(kTileBytes >= 3000 * sizeof(float2), "the tail's right-hand sides fit (a tail has fewer than 3000 cells)");
+extern __shared__ __align__(16) unsigned char dyn_smem[];
+DEV Tail make_tail(const DevScene& d) {
+    const Lv F = lev(d.lv, d.lv.tail), E = lev(d.lv, d.lv.n - 1);
+    return tail_at(dyn_smem + kTileBytes, reinterpret_cast<float2*>(dyn_smem), F.off, E.off + E.w * E.h - F.off, F.w * F.h,
+                   d.lv.n - d.lv.tail);
 }
-// The first tail level's cells (a batch keeps their couplings out of shared memory).
-__host__ __device__ inline int tail_first_cells(const Levels& lv) { return lv.w[lv.tail] * lv.h[lv.tail]; }
+
+// Cells of the tail levels, and the tail's bytes without its right-hand sides.
+__host__ __device__ inline int tail_cells(const Levels& lv) { return lv.off[lv.n - 1] + lv.w[lv.n - 1] * lv.h[lv.n - 1] - lv.off[lv.tail]; }
+__host__ __device__ inline size_t tail_bytes(int T) {
+    return (kTailLevels * sizeof(TailLevel) + (size_t)T * (sizeof(float4) + 2 * sizeof(float2) + 2 * sizeof(uint16_t)) + 15) / 16 * 16;
+}
 
 // mg_tail.comp mode 1 in every block's shared memory, once per solve: the first tail
 // level's matrix from global memory, then the Galerkin matrices of the coarser tail levels
 // (the arithmetic of mg_build.comp). Block 0 also stores them for inspection.
 template <class M>
 DEV void tail_setup(const DevScene& d, const Tail& tl, bool writer) {
+    if (threadIdx.x < (uint32_t)tl.nl) {
+        const Lv L = lev(d.lv, d.lv.tail + threadIdx.x);
+        tl.lv[threadIdx.x] = TailLevel{L.off - tl.base, L.w * L.h, L.w, L.h, L.wm, 0, 0, 0};
+    }
     for (int s = threadIdx.x; s < tl.nf; s += NT) {
-        if (s >= tl.aoff) tl.a[s - tl.aoff] = M::A(d, tl.base + s);
-        tl.dg[s] = M::Dg(d, tl.base + s);
+        tl.a[s] = M::A(d, tl.base + s);
+        tl.dy[s].x = M::Dg(d, tl.base + s);
     }
     __syncthreads();
     for (int l = d.lv.tail; l < d.lv.n - 1; l++) {
@@ -400,8 +407,8 @@ DEV void tail_setup(const DevScene& d, const Tail& tl, bool writer) {
                 int cx = 2 * ccx + (k & 1), cy = 2 * ccy + (k >> 1);
                 if (!t_unknown(tl, F, cx, cy)) continue;
                 int i = o + cy * F.w + cx;
-                D += tl.dg[i];
-                float4 w = tail_a<M>(d, tl, i);
+                D += tl.dy[i].x;
+                float4 w = tl.a[i];
                 for (int q = 0; q < 4; q++) {
                     int nx = cx + NBX[q], ny = cy + NBY[q];
                     if (!t_unknown(tl, F, nx, ny)) continue;
@@ -413,72 +420,81 @@ DEV void tail_setup(const DevScene& d, const Tail& tl, bool writer) {
                     else A.w += wd;
                 }
             }
-            tl.dg[oc + t] = D > 1e-7f ? D : 0.0f;
-            tl.a[oc + t - tl.aoff] = D > 1e-7f ? A : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            if (writer) M::setA(d, C.off + t, tl.a[oc + t - tl.aoff], tl.dg[oc + t]);
+            tl.dy[oc + t].x = D > 1e-7f ? D : 0.0f;
+            tl.a[oc + t] = D > 1e-7f ? A : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if (writer) M::setA(d, C.off + t, tl.a[oc + t], tl.dy[oc + t].x);
         }
         __syncthreads();
     }
-    // the unknowns around every tail cell, for the sweeps
-    for (int l = d.lv.tail; l < d.lv.n; l++) {
-        const Lv L = lev(d.lv, l);
-        const int o = L.off - tl.base;
-        for (int t = threadIdx.x; t < L.w * L.h; t += NT) {
-            const int y = qdiv(t, L.wm), x = t - y * L.w;
-            uint32_t m = tl.dg[o + t] > 0.0f ? 16u : 0u;
-            for (int q = 0; q < 4; q++) m |= t_unknown(tl, L, x + NBX[q], y + NBY[q]) ? (1u << q) : 0u;
-            tl.m[o + t] = (uint8_t)m;
+    // the lists (an entry's place among its colour does not matter to a half-sweep): the couplings
+    // and diagonals so far lie by slot, so they move through registers, level by level
+    for (int l = 0; l < tl.nl; l++) {
+        const Lv L = lev(d.lv, d.lv.tail + l);
+        TailLevel& Q = tl.lv[l];
+        constexpr int PER = 6;   // a first tail level has at most 1500 cells
+        float4 a[PER];
+        float2 dy[PER];
+        int p[PER];
+        for (int j = 0; j < PER; j++) {
+            const int t = threadIdx.x + j * NT;
+            if (t >= Q.n) break;
+            const int y = qdiv(t, L.wm), x = t - y * L.w, s = Q.o + t;
+            a[j] = tl.a[s];
+            dy[j] = make_float2(tl.dy[s].x, recip(tl.dy[s].x));
+            if (!t_unknown(tl, L, x - 1, y)) a[j].x = 0.0f;
+            if (!t_unknown(tl, L, x + 1, y)) a[j].y = 0.0f;
+            if (!t_unknown(tl, L, x, y - 1)) a[j].z = 0.0f;
+            if (!t_unknown(tl, L, x, y + 1)) a[j].w = 0.0f;
+            p[j] = -1;
+            if (dy[j].x > 0.0f) p[j] = ((x + y) & 1) ? Q.n - 1 - atomicAdd(&Q.n1, 1) : atomicAdd(&Q.n0, 1);
+            tl.x[s] = make_float2(0.0f, 0.0f);
+        }
+        __syncthreads();
+        const int gap = Q.n - Q.n1 - Q.n0;   // the odd cells, so far at the list's end, follow the even ones
+        for (int j = 0; j < PER; j++) {
+            const int t = threadIdx.x + j * NT;
+            if (t >= Q.n) break;
+            int e = p[j];
+            if (e >= Q.n0) e -= gap;
+            tl.ent[Q.o + t] = e < 0 ? (uint16_t)kNoEntry : (uint16_t)(Q.o + e);
+            if (e < 0) continue;
+            tl.a[Q.o + e] = a[j];
+            tl.dy[Q.o + e] = dy[j];
+            tl.slot[Q.o + e] = (uint16_t)(Q.o + t);
         }
     }
     __syncthreads();
 }
 
-// Where a way up reads the coarse level's finished values: this block's shared copy of the
-// first tail level (s), or the level in global memory through M (at offset off).
-struct Zc {
-    const float2* s;
-    int off, w;
-};
-
-// A level's tile and RH cells around it staged in shared memory, RW x RW slots: the
-// diagonal (zero outside the level), the couplings, up to three vector fields, and for the
-// tile's own cells (one per thread) two more vectors and the operator's diagonal. A tile body
-// comes in two halves: stage_* issues every load of the tile as an asynchronous copy into a
-// Region (zero-filled outside the level), and finish_* runs once they have landed and reads
-// only the slots, each as the shader reads its field (a diagonal that is not positive as
-// zero, BF16 couplings widened, the fused residual update applied). Its values are the same,
-// value for value, as reading the fields from global memory one after another. Every block
-// holds two Regions: while one tile computes, the copies of its next tile are in flight
-// (pipe_active).
-constexpr int RH = 2;
-constexpr int RW = 16 + 2 * RH;
-constexpr int RN = RW * RW;
-struct Region {
-    float dg[RN];
-    float4 a[RN];
-    float2 u[RN], v[RN];
-    union {
-        float2 w[RN];   // a way up: each slot's coarse-grid value
-        struct {        // a way down fused with the CG update: the tile's own p, x and diagonal
-            float2 o1[NT], o2[NT];
-            float od[NT];
-        } o;
-    };
-    float2 ring[32];   // the black cells just outside the tile, once computed (ring_cell)
-};
-DEV int rslot(int lx, int ly) { return (ly + RH) * RW + lx + RH; }
-__constant__ int RSTEP[4] = {-1, 1, -RW, RW};
-
-// The cells of a tile by colour for the smoothing passes: threads 0 .. 127 take the red
-// cells ((x + y) even; tiles start at even coordinates), 128 .. 255 the black ones, eight to
-// a row, so that no warp holds both the short red formula and the long black one.
-DEV int2 colour_cell() {
-    const int c = threadIdx.x & 127, ly = c >> 3;
-    return make_int2(2 * (c & 7) + ((ly & 1) ^ (threadIdx.x < 128 ? 0 : 1)), ly);
-}
-// The 32 black cells just outside a tile that its red border cells touch: slot j of side
-// s = r / 8: (-1, 2j), (16, 2j + 1), (2j, -1), (2j + 1, 16); and the slot of such a cell.
-DEV int2 ring_cell(int r) {
+// ---- the level passes ---------------------------------------------------------------------------
+//
+// A block takes a 16 x 16 tile at a time, a thread per cell: warps 0-3 its black cells, warps
+// 4-7 its red ones, so that no warp mixes the two colours' formulas. What a smoothing pass
+// needs around the tile comes with it: the 32 black cells just outside it that its red border
+// cells touch are computed here too (warp 4), and the 66 red cells around those are read by
+// warps 5-7. A thread stages its own cell's fields one tile ahead by asynchronous copies into
+// slots only it reads (cp.async: waiting for a register load would also wait for the later ones
+// that share one of a warp's few scoreboards); what neighbours need goes through shared memory
+// by colour, each colour's slots contiguous (slot row ly + 2 of ten, column (lx + 2) / 2), so
+// that a warp's accesses do not conflict. Two block barriers a tile.
+//
+// A pass is bound by the latency of its steps, not by bytes (L2 carries 16 % of its peak): what
+// counts is how few instructions stand between a tile's arrival and its results, and that none
+// of them waits for memory. Against the pass this replaced (every thread staging and
+// reading up to 400 slots, ten IEEE divisions inlined per black cell, 250 KB of code in the
+// loop), per iteration of the 1024 x 576 full-physics pour, 7.6 tiles a block: way down on
+// level 0 18.5 -> 12.8 us, way up 15.4 -> 10.1, apply 11.4 -> 8.2, a coarse level with one tile a
+// block 2.3-3.0 -> 1.7-2.0. Tried and slower: ten lanes of a warp marching up a tile without
+// block barriers (too few warps to hide its ~1000 instructions a row pair: 19 / 12 / 13 us).
+//
+// The values are those of the shaders' work groups, term by term in their order. A neighbour
+// that is no unknown is a term less there; here its value is -0 (or, where the term is
+// subtracted, +0), which adds nothing to any sum.
+constexpr int SP = 10;   // slots of a row
+DEV int slot_of(int lx, int ly) { return (ly + 2) * SP + ((lx + 2) >> 1); }
+// The 32 black cells just outside a tile that its red border cells touch: (-1, 2j), (16, 2j + 1),
+// (2j, -1), (2j + 1, 16).
+DEV int2 ring_black(int r) {
     const int j = r & 7;
     switch (r >> 3) {
         case 0: return make_int2(-1, 2 * j);
@@ -487,426 +503,657 @@ DEV int2 ring_cell(int r) {
         default: return make_int2(2 * j + 1, 16);
     }
 }
-DEV int ring_of(int lnx, int lny) {
-    if (lnx < 0) return lny >> 1;
-    if (lnx > 15) return 8 + (lny >> 1);
-    if (lny < 0) return 16 + (lnx >> 1);
-    return 24 + (lnx >> 1);
-}
-
-// The slots of a region that thread threadIdx.x copies and makes final: k = threadIdx.x +
-// j NT (j < RJ), at cell (ox - RH + k % RW, oy - RH + k / RW) of the level.
-constexpr int RJ = (RN + NT - 1) / NT;
-
-// This block's work items through the pipeline of solve_common.cuh with kDepth regions:
-// stage(it, rg) issues item it's copies into a region, finish(it, rg) computes it.
-constexpr int kDepth = 2;
-template <class I, class S, class F>
-DEV void pipe_tiles(uint32_t cnt, I&& item, Region* rg, S&& stage, F&& finish) {
-    pipeline<kDepth>(cnt, item, [&](uint32_t it, int b) { stage(it, rg[b]); }, [&](uint32_t it, int b) { finish(it, rg[b]); });
-}
-
-template <class M>
-DEV float2 coarse_z(const DevScene& d, const Zc& zc, int mx, int my) {
-    const int k = (my >> 1) * zc.w + (mx >> 1);
-    return zc.s ? zc.s[k] : M::Z(d, zc.off + k);
-}
-
-// mg_down.comp on tile t of level l, copies: the diagonal, the couplings, the right-hand
-// side (level 0: the residual before the update, and q when R.q) over the region; with
-// `update` (level 0 fused with cg_update.comp) the tile's own p, x and operator diagonal.
-template <class M>
-DEV void stage_down(const DevScene& d, const Lv& F, int t, const Rsrc<M>& R, bool update, const float2* p, Region& rg) {
-    const int2 og = tile_origin(F, t);
-    const int ox = og.x, oy = og.y;
-    const float2* r = R.r ? R.r : d.mgr;
-#pragma unroll
-    for (int j = 0; j < RJ; j++) {
-        const int k = threadIdx.x + j * NT;
-        if (k >= RN) break;
-        const int x = ox - RH + k % RW, y = oy - RH + k / RW;
-        const bool in = l_inside(F, x, y);
-        const int i = in ? l_at(F, x, y) : 0;
-        cp_async<4>(&rg.dg[k], M::Dptr(d) + i, in);
-        cp_async<M::kABytes>(&rg.a[k], M::Araw(d, i), in);
-        cp_async<8>(&rg.u[k], r + i, in);
-        if (R.q) cp_async<8>(&rg.v[k], R.q + i, in);
-    }
-    if (update) {
-        const int cx = ox + (threadIdx.x & 15), cy = oy + (threadIdx.x >> 4);
-        const bool in = l_inside(F, cx, cy);
-        const int i = in ? l_at(F, cx, cy) : 0;
-        cp_async<4>(&rg.o.od[threadIdx.x], d.mgd + i, in);
-        cp_async<8>(&rg.o.o1[threadIdx.x], p + i, in);
-        cp_async<8>(&rg.o.o2[threadIdx.x], d.pres + i, in);
+// The 66 red cells around the tile that those and the tile's black cells touch: 32 beside it,
+// 32 one further out, two corners.
+DEV int2 ring_red(int r) {
+    const int j = r & 7;
+    switch (r >> 3) {
+        case 0: return make_int2(-1, 2 * j + 1);
+        case 1: return make_int2(16, 2 * j);
+        case 2: return make_int2(2 * j + 1, -1);
+        case 3: return make_int2(2 * j, 16);
+        case 4: return make_int2(-2, 2 * j);
+        case 5: return make_int2(17, 2 * j + 1);
+        case 6: return make_int2(2 * j, -2);
+        case 7: return make_int2(2 * j + 1, 17);
+        default: return j == 0 ? make_int2(-1, -1) : make_int2(16, 16);
     }
 }
+// A thread's cell of the tile and its slot (left neighbour's slot: s - e, right: s - e + 1,
+// below: s - SP, above: s + SP), and its cell of the ring: kind 1 black, 2 red, 0 none.
+struct Geo {
+    int lx, ly, s, e;
+    int ex, ey, es, ee, kind;
+    bool red;
+};
+DEV Geo geo() {   // (once per kernel: the passes take it)
+    Geo g;
+    const int t = threadIdx.x, u = t & 127;
+    g.red = t >= 128;
+    g.ly = u >> 3;
+    g.lx = 2 * (u & 7) + ((g.ly & 1) ^ (g.red ? 0 : 1));
+    g.s = slot_of(g.lx, g.ly);
+    g.e = 1 - (g.lx & 1);
+    g.kind = t < 128 ? 0 : t < 160 ? 1 : t < 226 ? 2 : 0;
+    const int2 c = g.kind == 1 ? ring_black(t - 128) : g.kind == 2 ? ring_red(t - 160) : make_int2(0, 0);
+    g.ex = c.x;
+    g.ey = c.y;
+    g.es = slot_of(c.x, c.y);
+    g.ee = 1 - (c.x & 1);
+    return g;
+}
 
-// ... and its arithmetic. On level 0 with `r_out` it also applies cg_update.comp: x +=
-// alpha p and the residual update into r_out. The staged slots are read as the shader reads
-// its fields: a diagonal that is not positive as zero (dg), the right-hand side with the fused
-// update (rhs). Every neighbour's values are read before the terms are summed, in the
-// shader's order, each kept or not by a select.
-template <class M>
-DEV void finish_down(const DevScene& d, const Lv& F, const Lv& C, int t, const Rsrc<M>& R, float2* r_out, float2* sz,
-                     Region& rg) {
-    const int2 og = tile_origin(F, t);
-    const int ox = og.x, oy = og.y;
-    __syncthreads();   // (every thread's copies have landed)
-    const bool fused = R.q != nullptr;
-    auto dg = [&](int k) {
-        const float v = rg.dg[k];
-        return v > 0.0f ? v : 0.0f;
+DEV float2 f2sel(bool c, float2 a, float z) { return make_float2(c ? a.x : z, c ? a.y : z); }
+DEV float2 mul2(float w, float2 v) { return make_float2(w * v.x, w * v.y); }
+// r + t0 + t1 + t2 + t3 (left, right, below, above)
+DEV float2 sum4(float2 r, float2 t0, float2 t1, float2 t2, float2 t3) {
+    float2 s = r;
+    s.x += t0.x; s.y += t0.y;
+    s.x += t1.x; s.y += t1.y;
+    s.x += t2.x; s.y += t2.y;
+    s.x += t3.x; s.y += t3.y;
+    return s;
+}
+
+// The tree of reduce.glsl:5-14 over a tile's 256 products (cell ly * 16 + lx), by one warp: the
+// tree's row steps of a column by its two lanes, then the column steps by shuffles; the sum
+// comes out in lane 0.
+DEV float2 tile_tree(const float2* v) {
+    const int x = threadIdx.x & 15, h = (threadIdx.x >> 4) & 1;
+    auto b = [&](int j) {
+        const float2 v0 = v[j * 16 + x], v1 = v[(j + 4) * 16 + x], v2 = v[(j + 8) * 16 + x], v3 = v[(j + 12) * 16 + x];
+        return make_float2((v0.x + v2.x) + (v1.x + v3.x), (v0.y + v2.y) + (v1.y + v3.y));
     };
-    auto rhs = [&](int k) {   // R.at: r - alpha q
-        float2 v = rg.u[k];
+    const float2 b0 = b(h), b1 = b(h + 2);
+    float2 s = make_float2(b0.x + b1.x, b0.y + b1.y);
+#pragma unroll
+    for (int k = 16; k > 0; k >>= 1) {
+        s.x += __shfl_down_sync(0xffffffffu, s.x, k);
+        s.y += __shfl_down_sync(0xffffffffu, s.y, k);
+    }
+    return s;
+}
+constexpr int kTreeWarp = 7;
+
+// A tile's fields as they are staged: thread t's own cell in entry t, its cell of the ring in
+// entry t - 128 of the e arrays.
+template <class M>
+struct LevelStage {
+    typename M::Row a[NT], ea[32];
+    float2 r[NT], er[98], q[NT], eq[98], p[NT], x[NT];
+    typename M::Diag y[NT], ey[98];
+};
+static_assert(sizeof(LevelStage<Plain>) <= sizeof(TileSmem::stage) / 2, "two tiles' fields");
+struct ApplyStage {
+    float4 a[NT];
+    float2 z[NT], o[NT], ez[64], eo[64];
+    float D[NT], eD[64];
+};
+
+// A tile of a level of a scene as a pass works on it.
+struct DownArgs {
+    const float2 *r, *q;   // the right-hand side; on level 0 fused with cg_update.comp, A p (else null)
+    float ax, ay;          // ... and its step lengths,
+    const float2* p;       // the directions,
+    float2* r_out;         // and where the updated residual goes
+};
+struct DownTile {
+    int scene;
+    Lv F, C;
+    int t;
+    DownArgs a;
+};
+
+// mg_down.comp on this block's tiles of a level (at(k): its k-th, first and next(k): the indices it
+// takes): red-black Gauss-Seidel from zero, the residual summed over 2 x 2 cells into the next
+// level. On level 0 (top) also the tile's sums of r.r into part[tile].zw (the way up adds those
+// of r.z) and, where q is set, x += alpha p, r -= alpha q (a cell that is no unknown has p = 0,
+// and what its r holds is never used). True if an operand left the fast quotients' range.
+template <class M, bool SLOW, class Of, class At, class Next>
+DEV bool down_pass_(const Geo& g, int count, bool top, Of&& of, At&& at, Next&& next) {
+    TileSmem& S = *reinterpret_cast<TileSmem*>(dyn_smem);
+    const int t = threadIdx.x;
+    bool bad = false;
+    using Stage = LevelStage<M>;
+    auto fetch = [&](const DownTile& T, Stage& n) {
+        const DevScene& d = of(T.scene);
+        const int2 og = tile_origin(T.F, T.t);
+        const int x = og.x + g.lx, y = og.y + g.ly;
+        const bool in = x < T.F.w && y < T.F.h;
+        const int i = in ? l_at(T.F, x, y) : 0;
+        cp_async<sizeof(typename M::Row)>(&n.a[t], M::rows(d) + i, in);
+        cp_async<sizeof(typename M::Diag)>(&n.y[t], M::diags(d) + i, in);
+        cp_async<8>(&n.r[t], T.a.r + i, in);
+        if (T.a.q) {
+            cp_async<8>(&n.q[t], T.a.q + i, in);
+            cp_async<8>(&n.p[t], T.a.p + i, in);
+            cp_async<8>(&n.x[t], d.pres + i, in);
+        }
+        if (g.kind != 0) {
+            const int ex = og.x + g.ex, ey = og.y + g.ey;
+            const bool ein = l_inside(T.F, ex, ey);
+            const int e = ein ? l_at(T.F, ex, ey) : 0;
+            cp_async<sizeof(typename M::Diag)>(&n.ey[t - 128], M::diags(d) + e, ein);
+            cp_async<8>(&n.er[t - 128], T.a.r + e, ein);
+            if (T.a.q) cp_async<8>(&n.eq[t - 128], T.a.q + e, ein);
+            if (g.kind == 1) cp_async<sizeof(typename M::Row)>(&n.ea[t - 128], M::rows(d) + e, ein);
+        }
+    };
+    auto stage = [](int turn) -> Stage& { return *reinterpret_cast<Stage*>(dyn_smem + (turn & 1) * sizeof(TileSmem::stage) / 2); };
+    int k = next(0);
+    if (k >= count) return false;
+    DownTile T = at(k);
+    fetch(T, stage(0));
+    cp_commit();
+    for (int turn = 0;; turn++) {
+        const DownTile cur = T;
+        k = next(k + 1);
+        const bool more = k < count;
+        if (more) {
+            T = at(k);
+            fetch(T, stage(turn + 1));
+        }
+        cp_commit();
+        cp_wait<1>();
+        const Stage& n = stage(turn);
+        const int2 og = tile_origin(cur.F, cur.t);
+        const bool fused = cur.a.q != nullptr, in = og.x + g.lx < cur.F.w && og.y + g.ly < cur.F.h;
+        const int i = l_at(cur.F, og.x + g.lx, og.y + g.ly);
+        const typename M::Diag y = n.y[t];
+        typename M::Diag ey = M::no_diag();
+        float2 r = n.r[t], er = make_float2(0.0f, 0.0f);
         if (fused) {
-            const float2 qq = rg.v[k];
-            v.x = v.x - R.ax * qq.x;
-            v.y = v.y - R.ay * qq.y;
-        }
-        return v;
-    };
-    // the value of black slot k after the half-sweep from zero (mg_down black())
-    auto black = [&](int k) {
-        const float4 w = M::Aslot(rg.a[k]);
-        float2 sum = rhs(k);
-        const float d0 = dg(k - 1), d1 = dg(k + 1), d2 = dg(k - RW), d3 = dg(k + RW);
-        const float2 r0 = rhs(k - 1), r1 = rhs(k + 1), r2 = rhs(k - RW), r3 = rhs(k + RW);
-        const float t0x = M::quotp(w.x * r0.x, d0), t0y = M::quotp(w.x * r0.y, d0);
-        const float t1x = M::quotp(w.y * r1.x, d1), t1y = M::quotp(w.y * r1.y, d1);
-        const float t2x = M::quotp(w.z * r2.x, d2), t2y = M::quotp(w.z * r2.y, d2);
-        const float t3x = M::quotp(w.w * r3.x, d3), t3y = M::quotp(w.w * r3.y, d3);
-        if (d0 > 0.0f) { sum.x += t0x; sum.y += t0y; }
-        if (d1 > 0.0f) { sum.x += t1x; sum.y += t1y; }
-        if (d2 > 0.0f) { sum.x += t2x; sum.y += t2y; }
-        if (d3 > 0.0f) { sum.x += t3x; sum.y += t3y; }
-        return M::quot(sum, dg(k));
-    };
-    // one cell's z (mg_down: red from zero, black after it), the CG update and mgx
-    auto own = [&](int lx, int ly, bool red) {
-        const int cell = ly * 16 + lx;
-        const int cx = ox + lx, cy = oy + ly;
-        const int k0 = rslot(lx, ly);
-        float2 z = make_float2(0.0f, 0.0f);
-        if (l_inside(F, cx, cy)) {
-            const int i = l_at(F, cx, cy);
-            const float D = dg(k0);
-            if (D > 0.0f) {
-                if (red) {
-                    z = M::quot(rhs(k0), D);
-                } else {
-                    z = black(k0);
-                }
+            const float2 q = n.q[t], p = n.p[t], x = n.x[t];
+            r.x = r.x - cur.a.ax * q.x;
+            r.y = r.y - cur.a.ay * q.y;
+            if (in) {
+                if (!SLOW) of(cur.scene).pres[i] = make_float2(x.x + cur.a.ax * p.x, x.y + cur.a.ay * p.y);   // (once)
+                cur.a.r_out[i] = r;
             }
-            if (r_out && rg.o.od[cell] > 0.0f) {
-                // cg_update.comp: x += alpha p, r -= alpha q (unknowns of active tiles)
-                const float2 pp = rg.o.o1[cell];
-                float2 x = rg.o.o2[cell];
-                x.x += R.ax * pp.x;
-                x.y += R.ay * pp.y;
-                d.pres[i] = x;
-                r_out[i] = rhs(k0);
+        }
+        if (g.kind != 0) {
+            ey = n.ey[t - 128];
+            er = n.er[t - 128];
+            if (fused) {
+                const float2 eq = n.eq[t - 128];
+                er.x = er.x - cur.a.ax * eq.x;
+                er.y = er.y - cur.a.ay * eq.y;
             }
-            M::setX(d, i, z);
         }
-        sz[cell] = z;
-    };
-    // warps 0-3: the 128 black cells; warp 4: the 32 black cells around the tile (ring_cell),
-    // which the restriction needs; warps 5-7: the 128 red cells (the shorter formula), 96 + 32
-    const int tid = threadIdx.x;
-    if (tid < 128) {
-        const int ly = tid >> 3;
-        own(2 * (tid & 7) + 1 - (ly & 1), ly, false);
-    } else if (tid < 160) {
-        const int2 rc = ring_cell(tid - 128);
-        const int kr = rslot(rc.x, rc.y);
-        rg.ring[tid - 128] = dg(kr) > 0.0f ? black(kr) : make_float2(0.0f, 0.0f);
-    } else {
-        for (int c = tid - 160; c < 128; c += 96) {
-            const int ly = c >> 3;
-            own(2 * (c & 7) + (ly & 1), ly, true);
+        const bool unk = M::unk(y), eunk = M::unk(ey);
+        if (top) S.prod[g.ly * 16 + g.lx] = f2sel(unk, make_float2(r.x * r.x, r.y * r.y), 0.0f);
+        r = f2sel(unk, r, -0.0f);
+        er = f2sel(eunk, er, -0.0f);
+        if (g.red) {
+            if (!SLOW) bad |= unk && !M::ok(r, y);
+            S.red[g.s] = M::pack_red(r, y);
+            if (in) of(cur.scene).mgx[i] = f2sel(unk, M::template quot<SLOW>(r, y), 0.0f);
+            if (g.kind == 2) {
+                if (!SLOW) bad |= eunk && !M::ok(er, ey);
+                S.red[g.es] = M::pack_red(er, ey);
+            }
         }
+        __syncthreads();
+        if (t < 160) {   // the black cells, and warp 4 those of the ring
+            const bool own = t < 128;
+            const int s = own ? g.s : g.es, e = own ? g.e : g.ee;
+            const float4 w = M::wide(own ? n.a[t] : n.ea[t - 128]);
+            const typename M::Diag yo = own ? y : ey;
+            auto term = [&](float wq, int j) {
+                float2 v;
+                typename M::Diag yn;
+                M::unpack_red(S.red[j], v, yn);
+                return M::template quot<SLOW>(mul2(wq, v), yn);
+            };
+            const float2 sum = sum4(own ? r : er, term(w.x, s - e), term(w.y, s - e + 1), term(w.z, s - SP), term(w.w, s + SP));
+            const bool u = own ? unk : eunk;
+            if (!SLOW) bad |= u && !M::ok(sum, yo);
+            const float2 z = f2sel(u, M::template quot<SLOW>(sum, yo), 0.0f);
+            S.black[s] = z;
+            if (own && in) of(cur.scene).mgx[i] = z;
+        } else if (top && t >= 32 * kTreeWarp) {
+            const float2 rr = tile_tree(S.prod);
+            if ((t & 31) == 0) reinterpret_cast<float2*>(M::part(of(cur.scene)) + cur.t)[1] = rr;
+        }
+        __syncthreads();
+        if (g.red) {   // the restriction: a coarse cell's red cells are in lanes l (even row) and l + 8
+            const float4 w = M::wide(n.a[t]);
+            const float2 t0 = mul2(w.x, S.black[g.s - g.e]), t1 = mul2(w.y, S.black[g.s - g.e + 1]);
+            const float2 t2 = mul2(w.z, S.black[g.s - SP]), t3 = mul2(w.w, S.black[g.s + SP]);
+            float2 s = f2sel(unk, sum4(make_float2(0.0f, 0.0f), t0, t1, t2, t3), 0.0f);
+            s.x = __shfl_up_sync(0xffffffffu, s.x, 8);
+            s.y = __shfl_up_sync(0xffffffffu, s.y, 8);
+            if (g.ly & 1) {
+                const float2 v = sum4(s, t0, t1, t2, t3);
+                s = unk ? v : s;
+                const int X = (og.x + g.lx) >> 1, Y = (og.y + g.ly) >> 1;
+                if (X < cur.C.w && Y < cur.C.h) of(cur.scene).mgr[l_at(cur.C, X, Y)] = s;
+            }
+        }
+        if (!more) break;
     }
-    __syncthreads();
-    if (threadIdx.x < 64) {   // the restriction: aggregate (ax, ay), its red cells (0, 0) and (1, 1)
-        const int ax = threadIdx.x & 7, ay = threadIdx.x >> 3;
-        const int Cx = (ox >> 1) + ax, Cy = (oy >> 1) + ay;
-        if (Cx < C.w && Cy < C.h) {
-            float sx = 0.0f, sy = 0.0f;
-#pragma unroll
-            for (int k = 0; k < 2; k++) {
-                const int lqx = 2 * ax + k, lqy = 2 * ay + k;
-                const int kq = rslot(lqx, lqy);
-                const bool own = dg(kq) > 0.0f;
-                const float4 w = M::Aslot(rg.a[kq]);
-                float dn[4];
-                float2 zb[4];
-#pragma unroll
-                for (int q = 0; q < 4; q++) {
-                    dn[q] = dg(kq + RSTEP[q]);
-                    const int lnx = lqx + NBX[q], lny = lqy + NBY[q];
-                    const bool here = lnx >= 0 && lny >= 0 && lnx < 16 && lny < 16;
-                    zb[q] = here ? sz[lny * 16 + lnx] : rg.ring[ring_of(lnx, lny)];
-                }
-#pragma unroll
-                for (int q = 0; q < 4; q++) {
-                    const float wd = wcomp(w, q);
-                    const float ux = wd * zb[q].x, uy = wd * zb[q].y;
-                    if (own && dn[q] > 0.0f) {
-                        sx += ux;
-                        sy += uy;
-                    }
-                }
-            }
-            M::setR(d, l_at(C, Cx, Cy), make_float2(sx, sy));
-        }
-    }
-    __syncthreads();
+    return bad;
 }
-
-// mg_up.comp on tile t of level l, copies: the diagonal, the couplings, the right-hand side
-// (u), the pre-smoothed values mgx (v) and each slot's coarse-grid value (w; from zc.s, this
-// block's shared copy of the tail, in finish_up).
-template <class M>
-DEV void stage_up(const DevScene& d, const Lv& F, int t, const Rsrc<M>& rhs, const Zc& zc, Region& rg) {
-    const int2 og = tile_origin(F, t);
-    const int ox = og.x, oy = og.y;
-    const float2* r = rhs.r ? rhs.r : d.mgr;
-#pragma unroll
-    for (int j = 0; j < RJ; j++) {
-        const int k = threadIdx.x + j * NT;
-        if (k >= RN) break;
-        const int x = ox - RH + k % RW, y = oy - RH + k / RW;
-        const bool in = l_inside(F, x, y);
-        const int i = in ? l_at(F, x, y) : 0;
-        cp_async<4>(&rg.dg[k], M::Dptr(d) + i, in);
-        cp_async<M::kABytes>(&rg.a[k], M::Araw(d, i), in);
-        cp_async<8>(&rg.u[k], r + i, in);
-        cp_async<8>(&rg.v[k], d.mgx + i, in);
-        if (!zc.s) cp_async<8>(&rg.w[k], d.mgz + (in ? zc.off + (y >> 1) * zc.w + (x >> 1) : 0), in);
+// The tiles of a pass in which a fast quotient met an operand out of range are taken again by
+// the whole block with IEEE divisions: everything a pass writes comes out of its inputs (but x,
+// which only the first updates), so taking it twice is the same as once.
+template <class M, class Of, class At, class Next>
+DEV void down_pass(const Geo& g, int count, bool top, Of&& of, At&& at, Next&& next) {
+    if (count == 0) return;
+    const bool bad = down_pass_<M, false>(g, count, top, of, at, next);
+    if constexpr (!M::kMixed) {
+        if (__syncthreads_or(bad)) down_pass_<M, true>(g, count, top, of, at, next);
     }
 }
 
-// ... and its arithmetic; on level 0 (flag) the tile's sums of r.z, r.r into part[t]. Read
-// as finish_down reads its slots.
-template <class M>
-DEV void finish_up(const DevScene& d, const Lv& F, int t, bool flag, const Zc& zc, float2* sz, typename M::acc4* buf,
-                   Region& rg) {
-    using acc = typename M::acc;
-    typename M::acc4* part = M::part(d);
-    const int2 og = tile_origin(F, t);
-    const int ox = og.x, oy = og.y;
-    if (zc.s) {   // the coarse values from this block's copy of the tail
-#pragma unroll
-        for (int j = 0; j < RJ; j++) {
-            const int k = threadIdx.x + j * NT;
-            if (k >= RN) break;
-            const int x = ox - RH + k % RW, y = oy - RH + k / RW;
-            rg.w[k] = l_inside(F, x, y) ? coarse_z<M>(d, zc, x, y) : make_float2(0.0f, 0.0f);
+struct UpTile {
+    int scene;
+    Lv F, C;
+    int t;
+    const float2* r;    // the right-hand side
+    const float2* zc;   // the coarse level's values in global memory,
+    const float2* zs;   // or (else null) this block's copy of the tail in shared memory
+};
+
+// mg_up.comp on this block's tiles of a level: the coarse correction with omega and the
+// mirrored sweep. On level 0 (top) the tile's sums of r.z into part[tile].xy.
+template <class M, bool SLOW, class Of, class At, class Next>
+DEV bool up_pass_(const Geo& g, int count, bool top, Of&& of, At&& at, Next&& next) {
+    TileSmem& S = *reinterpret_cast<TileSmem*>(dyn_smem);
+    float2* const sred = reinterpret_cast<float2*>(S.red);
+    const int t = threadIdx.x;
+    bool bad = false;
+    using Stage = LevelStage<M>;   // (q: the pre-smoothed values, p and x: the coarse values of the tile and the ring)
+    auto fetch = [&](const UpTile& T, Stage& n) {
+        const DevScene& d = of(T.scene);
+        const int2 og = tile_origin(T.F, T.t);
+        const int x = og.x + g.lx, y = og.y + g.ly;
+        const bool in = x < T.F.w && y < T.F.h;
+        const int i = in ? l_at(T.F, x, y) : 0;
+        cp_async<sizeof(typename M::Row)>(&n.a[t], M::rows(d) + i, in);
+        cp_async<sizeof(typename M::Diag)>(&n.y[t], M::diags(d) + i, in);
+        cp_async<8>(&n.r[t], T.r + i, in);
+        if (g.red) {
+            cp_async<8>(&n.q[t], d.mgx + i, in);
+            if (!T.zs) cp_async<8>(&n.p[t], T.zc + (in ? (y >> 1) * T.C.w + (x >> 1) : 0), in);
         }
-    }
-    __syncthreads();
-    auto dg = [&](int k) {
-        const float v = rg.dg[k];
-        return v > 0.0f ? v : 0.0f;
-    };
-    // the new value of black slot k after the coarse correction (mg_up black())
-    auto black = [&](int k) {
-        const float4 w = M::Aslot(rg.a[k]);
-        float2 sum = rg.u[k];
-        float dn[4];
-        float2 xm[4], zcv[4];
-#pragma unroll
-        for (int q = 0; q < 4; q++) {
-            const int j = k + RSTEP[q];
-            dn[q] = dg(j);
-            xm[q] = rg.v[j];
-            zcv[q] = rg.w[j];
-        }
-#pragma unroll
-        for (int q = 0; q < 4; q++) {
-            const float wd = wcomp(w, q);
-            const float ux = wd * (xm[q].x + MG_OMEGA * zcv[q].x), uy = wd * (xm[q].y + MG_OMEGA * zcv[q].y);
-            if (dn[q] > 0.0f) {
-                sum.x += ux;
-                sum.y += uy;
+        if (g.kind != 0) {
+            const int ex = og.x + g.ex, ey = og.y + g.ey;
+            const bool ein = l_inside(T.F, ex, ey);
+            const int e = ein ? l_at(T.F, ex, ey) : 0;
+            cp_async<sizeof(typename M::Diag)>(&n.ey[t - 128], M::diags(d) + e, ein);
+            if (g.kind == 1) {
+                cp_async<sizeof(typename M::Row)>(&n.ea[t - 128], M::rows(d) + e, ein);
+                cp_async<8>(&n.er[t - 128], T.r + e, ein);
+            } else {
+                cp_async<8>(&n.eq[t - 128], d.mgx + e, ein);
+                if (!T.zs) cp_async<8>(&n.x[t - 128], T.zc + (ein ? (ey >> 1) * T.C.w + (ex >> 1) : 0), ein);
             }
         }
-        return M::quot(sum, dg(k));
     };
-    const int2 lc = colour_cell();
-    const int lx = lc.x, ly = lc.y, cell = ly * 16 + lx;
-    const int cx = ox + lx, cy = oy + ly;
-    const int k0 = rslot(lx, ly);
-    const bool red = threadIdx.x < 128;
-    const bool unk = dg(k0) > 0.0f;
-    float2 z = make_float2(0.0f, 0.0f);
-    if (unk && !red) z = black(k0);
-    sz[cell] = z;
-    if (threadIdx.x < 32) {   // (a red warp, idle here) the black cells around the tile
-        const int2 rc = ring_cell(threadIdx.x);
-        const int kr = rslot(rc.x, rc.y);
-        rg.ring[threadIdx.x] = dg(kr) > 0.0f ? black(kr) : make_float2(0.0f, 0.0f);
+    // s / D where the cell is an unknown
+    auto value = [&](float2 s, const typename M::Diag& y) {
+        if (!SLOW) bad |= M::unk(y) && !M::ok(s, y);
+        return M::template quot<SLOW>(s, y);
+    };
+    auto corrected = [](float2 v, float2 zc) { return make_float2(v.x + MG_OMEGA * zc.x, v.y + MG_OMEGA * zc.y); };
+    auto tree = [&](const UpTile& T) {
+        if (t < 32 * kTreeWarp) return;
+        const float2 rz = tile_tree(S.prod);
+        if ((t & 31) == 0) reinterpret_cast<float2*>(M::part(of(T.scene)) + T.t)[0] = rz;
+    };
+    auto stage = [](int turn) -> Stage& { return *reinterpret_cast<Stage*>(dyn_smem + (turn & 1) * sizeof(TileSmem::stage) / 2); };
+    int k = next(0);
+    if (k >= count) return false;
+    UpTile T = at(k);
+    fetch(T, stage(0));
+    cp_commit();
+    for (int turn = 0;; turn++) {
+        const UpTile cur = T;
+        k = next(k + 1);
+        const bool more = k < count;
+        if (more) {
+            T = at(k);
+            fetch(T, stage(turn + 1));
+        }
+        cp_commit();
+        cp_wait<1>();
+        const Stage& n = stage(turn);
+        const int2 og = tile_origin(cur.F, cur.t);
+        const int X = og.x + g.lx, Y = og.y + g.ly, i = l_at(cur.F, X, Y), cell = g.ly * 16 + g.lx;
+        const bool in = X < cur.F.w && Y < cur.F.h;
+        const typename M::Diag y = n.y[t];
+        typename M::Diag ey = M::no_diag();
+        if (g.kind != 0) ey = n.ey[t - 128];
+        const bool unk = M::unk(y), eunk = M::unk(ey);
+        const float2 r = n.r[t];
+        if (g.red) {
+            // (the tail's values are this block's own, in shared memory)
+            float2 zc = make_float2(0.0f, 0.0f);
+            if (unk) zc = cur.zs ? cur.zs[(Y >> 1) * cur.C.w + (X >> 1)] : n.p[t];
+            sred[g.s] = f2sel(unk, corrected(n.q[t], zc), -0.0f);
+            if (g.kind == 2) {
+                const int EX = og.x + g.ex, EY = og.y + g.ey;
+                float2 ez = make_float2(0.0f, 0.0f);
+                if (eunk) ez = cur.zs ? cur.zs[(EY >> 1) * cur.C.w + (EX >> 1)] : n.x[t - 128];
+                sred[g.es] = f2sel(eunk, corrected(n.eq[t - 128], ez), -0.0f);
+            }
+        }
+        __syncthreads();
+        if (t < 160) {   // the black cells, and warp 4 those of the ring
+            const bool own = t < 128;
+            const int s = own ? g.s : g.es, e = own ? g.e : g.ee;
+            const float4 w = M::wide(own ? n.a[t] : n.ea[t - 128]);
+            const typename M::Diag yo = own ? y : ey;
+            const float2 z = value(sum4(own ? r : n.er[t - 128], mul2(w.x, sred[s - e]), mul2(w.y, sred[s - e + 1]), mul2(w.z, sred[s - SP]),
+                                        mul2(w.w, sred[s + SP])), yo);
+            const bool u = own ? unk : eunk;
+            S.black[s] = f2sel(u, z, -0.0f);
+            if (own) {
+                if (in) of(cur.scene).mgz[i] = f2sel(u, z, 0.0f);
+                if (top) S.prod[cell] = f2sel(u, make_float2(r.x * z.x, r.y * z.y), 0.0f);
+            }
+        }
+        __syncthreads();
+        if (g.red) {
+            const float4 w = M::wide(n.a[t]);
+            const float2 z = value(sum4(r, mul2(w.x, S.black[g.s - g.e]), mul2(w.y, S.black[g.s - g.e + 1]), mul2(w.z, S.black[g.s - SP]),
+                                        mul2(w.w, S.black[g.s + SP])), y);
+            if (in) of(cur.scene).mgz[i] = f2sel(unk, z, 0.0f);
+            if (top) S.prod[cell] = f2sel(unk, make_float2(r.x * z.x, r.y * z.y), 0.0f);
+        }
+        if (top) {
+            __syncthreads();
+            tree(cur);
+        }
+        if (!more) break;
+    }
+    return bad;
+}
+template <class M, class Of, class At, class Next>
+DEV void up_pass(const Geo& g, int count, bool top, Of&& of, At&& at, Next&& next) {
+    if (count == 0) return;
+    const bool bad = up_pass_<M, false>(g, count, top, of, at, next);
+    if constexpr (!M::kMixed) {
+        if (__syncthreads_or(bad)) up_pass_<M, true>(g, count, top, of, at, next);
+    }
+}
+
+// cg_apply.comp on this block's level-0 tiles: p = z + beta p_old, q = A p (the FP32 operator),
+// the tile's sum of p.q into part[n + tile].zw. A thread per cell in row order, the 64 cells
+// beside the tile read by warps 4 and 5; the directions go through shared memory, two tiles in
+// flight, one block barrier a tile.
+struct ApplyTile {
+    int scene;
+    Lv F;
+    int t;
+    float b0, b1;
+    const float2* p_old;
+    float2* p_new;
+};
+template <class M, class Of, class At, class Next>
+DEV void apply_pass(int count, Of&& of, At&& at, Next&& next) {
+    if (count == 0) return;
+    TileSmem& S = *reinterpret_cast<TileSmem*>(dyn_smem);
+    constexpr int PW = 18;
+    static_assert(PW * PW * sizeof(float2) <= sizeof(S.red), "the directions in the red slots' bytes");
+    float2* const P = reinterpret_cast<float2*>(S.red);
+    const int t = threadIdx.x, lx = t & 15, ly = t >> 4;
+    const int hr = t - 128, hj = t & 15;   // the halo cell of threads 128 .. 191
+    const bool halo = t >= 128 && t < 192;
+    const int hx = hr < 16 ? -1 : hr < 32 ? 16 : hj, hy = hr < 32 ? hj : hr < 48 ? -1 : 16;
+    const int s0 = (ly + 1) * PW + lx + 1, sh = (hy + 1) * PW + hx + 1;
+    using Stage = ApplyStage;
+    auto nob = [](const ApplyTile& T) { return T.b0 == 0.0f && T.b1 == 0.0f; };
+    auto fetch = [&](const ApplyTile& T, Stage& n) {
+        const DevScene& d = of(T.scene);
+        const int2 og = tile_origin(T.F, T.t);
+        const int x = og.x + lx, y = og.y + ly;
+        const bool in = x < T.F.w && y < T.F.h;
+        const int i = in ? l_at(T.F, x, y) : 0;
+        cp_async<16>(&n.a[t], d.mga + i, in);
+        cp_async<4>(&n.D[t], d.mgd + i, in);
+        cp_async<8>(&n.z[t], d.mgz + i, in);
+        if (!nob(T)) cp_async<8>(&n.o[t], T.p_old + i, in);
+        if (halo) {
+            const int ex = og.x + hx, ey = og.y + hy;
+            const bool ein = l_inside(T.F, ex, ey);
+            const int e = ein ? l_at(T.F, ex, ey) : 0;
+            cp_async<4>(&n.eD[hr], d.mgd + e, ein);
+            cp_async<8>(&n.ez[hr], d.mgz + e, ein);
+            if (!nob(T)) cp_async<8>(&n.eo[hr], T.p_old + e, ein);
+        }
+    };
+    auto dir = [&](const ApplyTile& T, float2 z, float2 po, float D) {   // +0 where no unknown
+        float2 v = z;
+        if (!nob(T)) v = make_float2(T.b0 != 0.0f ? z.x + T.b0 * po.x : z.x, T.b1 != 0.0f ? z.y + T.b1 * po.y : z.y);
+        return f2sel(D > 0.0f, v, 0.0f);
+    };
+    auto stage = [](int slot) -> Stage& { return *reinterpret_cast<Stage*>(dyn_smem + slot * sizeof(Stage)); };
+    int slot = 0;   // this tile's stage
+    static_assert(3 * sizeof(Stage) <= sizeof(S.stage), "three tiles in flight");
+    int k = next(0);
+    if (k >= count) return;
+    ApplyTile T = at(k), T1 = T;
+    fetch(T, stage(0));
+    cp_commit();
+    k = next(k + 1);
+    if (k < count) {
+        T1 = at(k);
+        fetch(T1, stage(1));
+    }
+    cp_commit();
+    for (;;) {
+        const ApplyTile cur = T;
+        const bool more = k < count;   // (tile T1 is there)
+        T = T1;
+        if (more) k = next(k + 1);
+        if (more && k < count) {
+            T1 = at(k);
+            fetch(T1, stage(slot == 0 ? 2 : slot - 1));
+        }
+        cp_commit();
+        cp_wait<2>();
+        const Stage& n = stage(slot);
+        const int2 og = tile_origin(cur.F, cur.t);
+        const bool in = og.x + lx < cur.F.w && og.y + ly < cur.F.h;
+        const int i = l_at(cur.F, og.x + lx, og.y + ly);
+        const float D = n.D[t];
+        const float2 p = dir(cur, n.z[t], n.o[t], D);
+        P[s0] = p;
+        if (halo) P[sh] = dir(cur, n.ez[hr], n.eo[hr], n.eD[hr]);
+        __syncthreads();
+        const float4 a = n.a[t];
+        const float2 l = P[s0 - 1], r = P[s0 + 1], b = P[s0 - PW], u = P[s0 + PW];
+        float2 q = make_float2(D * p.x, D * p.y);
+        q.x -= a.x * l.x; q.y -= a.x * l.y;
+        q.x -= a.y * r.x; q.y -= a.y * r.y;
+        q.x -= a.z * b.x; q.y -= a.z * b.y;
+        q.x -= a.w * u.x; q.y -= a.w * u.y;
+        if (in) {
+            cur.p_new[i] = p;
+            of(cur.scene).cgq[i] = q;
+        }
+        S.prod[t] = f2sel(D > 0.0f, make_float2(p.x * q.x, p.y * q.y), 0.0f);
+        __syncthreads();
+        if (t >= 32 * kTreeWarp) {
+            const float2 pq = tile_tree(S.prod);
+            if ((t & 31) == 0) reinterpret_cast<float2*>(M::part(of(cur.scene)) + of(cur.scene).nwg + cur.t)[1] = pq;
+        }
+        if (!more) break;
+        slot = slot == 2 ? 0 : slot + 1;
+    }
+}
+
+// The tail's phases, over J cells a thread at once so that their chains overlap (past the end a
+// thread repeats the last one, whose value comes out the same).
+//
+// A half-sweep over entries p0 .. p0 + cnt - 1 of a level of width w.
+template <bool SLOW, int J>
+DEV void tail_sweep(const Tail& tl, int p0, int cnt, int w, bool& bad) {
+    if ((int)(threadIdx.x & ~31u) < cnt) {
+        int s[J];
+        float2 z[J];
+#pragma unroll
+        for (int j = 0; j < J; j++) {
+            const int p = p0 + min((int)threadIdx.x + j * NT, cnt - 1);
+            s[j] = tl.slot[p];
+            const float4 a = tl.a[p];
+            const float2 x0 = tl.x[max(s[j] - 1, 0)], x1 = tl.x[min(s[j] + 1, tl.T - 1)];
+            const float2 x2 = tl.x[max(s[j] - w, 0)], x3 = tl.x[min(s[j] + w, tl.T - 1)];
+            z[j] = quot2<SLOW>(sum4(tl.r[p], mul2(a.x, x0), mul2(a.y, x1), mul2(a.z, x2), mul2(a.w, x3)), tl.dy[p], bad);
+        }
+#pragma unroll
+        for (int j = 0; j < J; j++) tl.x[s[j]] = z[j];
     }
     __syncthreads();
-    typename M::acc4 a4 = M::zero4();
-    if (l_inside(F, cx, cy)) {
-        const int i = l_at(F, cx, cy);
-        if (unk) {
-            const float2 r = rg.u[k0];
-            if (red) {
-                const float4 w = M::Aslot(rg.a[k0]);
-                float dn[4];
-                float2 zb[4];
+}
+// The black half-sweep of a way up: its neighbours are read with their coarse correction.
+template <bool SLOW, int J>
+DEV void tail_correct(const Tail& tl, const TailLevel& L, const TailLevel& C, bool& bad) {
+    const int cnt = L.n1;
+    if ((int)(threadIdx.x & ~31u) < cnt) {
+        int s[J];
+        float2 z[J];
 #pragma unroll
-                for (int q = 0; q < 4; q++) {
-                    dn[q] = dg(k0 + RSTEP[q]);
-                    const int lnx = lx + NBX[q], lny = ly + NBY[q];
-                    const bool here = lnx >= 0 && lny >= 0 && lnx < 16 && lny < 16;
-                    zb[q] = here ? sz[lny * 16 + lnx] : rg.ring[ring_of(lnx, lny)];
-                }
-                float sx = r.x, sy = r.y;
-#pragma unroll
-                for (int q = 0; q < 4; q++) {
-                    const float wd = wcomp(w, q);
-                    const float ux = wd * zb[q].x, uy = wd * zb[q].y;
-                    if (dn[q] > 0.0f) {
-                        sx += ux;
-                        sy += uy;
-                    }
-                }
-                z = M::quot(make_float2(sx, sy), dg(k0));
-            }
-            a4 = M::prod4(r.x, z.x, r.y, z.y, r.x, r.x, r.y, r.y);
+        for (int j = 0; j < J; j++) {
+            const int p = L.o + L.n0 + min((int)threadIdx.x + j * NT, cnt - 1);
+            s[j] = tl.slot[p];
+            const float4 a = tl.a[p];
+            const int k = s[j] - L.o, y = qdiv(k, L.wm), x = k - y * L.w;
+            const int m = C.o + (y >> 1) * C.w + (x >> 1);
+            auto term = [&](float w, int sn, int c) {
+                const float2 xn = tl.x[min(max(sn, 0), tl.T - 1)], xc = tl.x[min(max(c, 0), tl.T - 1)];
+                return make_float2(w * (xn.x + MG_OMEGA * xc.x), w * (xn.y + MG_OMEGA * xc.y));
+            };
+            const float2 sum = sum4(tl.r[p], term(a.x, s[j] - 1, m - 1 + (x & 1)), term(a.y, s[j] + 1, m + (x & 1)),
+                                    term(a.z, s[j] - L.w, (y & 1) ? m : m - C.w), term(a.w, s[j] + L.w, (y & 1) ? m + C.w : m));
+            z[j] = quot2<SLOW>(sum, tl.dy[p], bad);
         }
-        M::setZ(d, i, z);
+#pragma unroll
+        for (int j = 0; j < J; j++) tl.x[s[j]] = z[j];
     }
-    if (flag) {
-        buf[cell] = a4;
-        block_tree(buf);
-        if (threadIdx.x == 0) part[t] = buf[0];
+    __syncthreads();
+}
+// The right-hand side of slot s of a tail level, and its first half-sweep, which starts from
+// zero: the level's even unknowns (entries below odd) are r / D. The odd ones are written before
+// anything reads them.
+template <bool SLOW>
+DEV void tail_rhs(const Tail& tl, int s, int odd, float2 r, bool& bad) {
+    const uint32_t p = tl.ent[s];
+    if (p == kNoEntry) return;
+    tl.r[p] = r;
+    if ((int)p < odd) tl.x[s] = quot2<SLOW>(r, tl.dy[p], bad);
+}
+// The residual of level L summed over the 2 x 2 cells of each cell of level C, four lanes to a
+// coarse cell, one per fine cell: a cell that is no unknown adds nothing (the sum is never -0,
+// so leaving it out or adding +0 is the same).
+template <bool SLOW>
+DEV void tail_restrict(const Tail& tl, const TailLevel& L, const TailLevel& C, bool& bad) {
+    const int cnt = 4 * C.n, k = threadIdx.x & 3, b = threadIdx.x & 28;
+#pragma unroll 1
+    for (int t = threadIdx.x; (t & ~31) < cnt; t += NT) {
+        const int c = min(t >> 2, C.n - 1), cy = qdiv(c, C.wm), cx = c - cy * C.w;
+        const int x = 2 * cx + (k & 1), y = 2 * cy + (k >> 1);
+        const bool in = x < L.w && y < L.h;
+        const int s = in ? L.o + y * L.w + x : L.o;
+        const uint32_t p = tl.ent[s];
+        const bool on = in && p != kNoEntry;
+        float2 e = make_float2(0.0f, 0.0f);
+        if (on) {
+            const float4 a = tl.a[p];
+            const float2 rh = tl.r[p], xs = tl.x[s];
+            const float D = tl.dy[p].x;
+            const float2 x0 = tl.x[max(s - 1, 0)], x1 = tl.x[min(s + 1, tl.T - 1)];
+            const float2 x2 = tl.x[max(s - L.w, 0)], x3 = tl.x[min(s + L.w, tl.T - 1)];
+            float2 z = make_float2(D * xs.x, D * xs.y);
+            z.x -= a.x * x0.x; z.y -= a.x * x0.y;
+            z.x -= a.y * x1.x; z.y -= a.y * x1.y;
+            z.x -= a.z * x2.x; z.y -= a.z * x2.y;
+            z.x -= a.w * x3.x; z.y -= a.w * x3.y;
+            e = make_float2(rh.x - z.x, rh.y - z.y);
+        }
+        float2 v = make_float2(0.0f, 0.0f);
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            v.x += __shfl_sync(0xffffffffu, e.x, b + q);
+            v.y += __shfl_sync(0xffffffffu, e.y, b + q);
+        }
+        if (k == 0 && t < cnt) tail_rhs<SLOW>(tl, C.o + c, C.o + C.n0, v, bad);
     }
     __syncthreads();
 }
 
 // mg_tail.comp mode 0, computed by EVERY block in its own shared memory: the V-cycle on the
-// tail levels, right-hand side the first tail level's mgr, result left in tl.x (the first
+// tail levels, right-hand side R (the first tail level's mgr), result left in tl.x (the first
 // tail level's slots). Every block gets the same values; the way up of the level above
 // reads them from its own copy, so no grid barrier follows the tail.
-template <class M>
-DEV void phase_tail(const DevScene& d, const Tail& tl, bool writer) {
-    const int first = d.lv.tail, last = d.lv.n - 1;
-    // Each level's first half-sweep starts from zero: its black cells are r / D, the rest 0.
-    // It is taken where the level's right-hand side is made (here for the first tail level,
-    // in the restriction for the others), which saves a pass and a barrier per level.
-    auto from_zero = [&](const Lv& L, int t, float2 r) {
-        const int y = qdiv(t, L.wm), x = t - y * L.w;
-        const int s = L.off - tl.base + t;
-        const float D = tl.dg[s];
-        if (!(D <= 0.0f) && ((x + y) & 1) == 0) tl.x[s] = divz(r, D);
-        else tl.x[s] = make_float2(0.0f, 0.0f);
-    };
-    {
-        const Lv F = lev(d.lv, first);
-        for (int s = threadIdx.x; s < tl.nf; s += NT) {
-            const float2 r = M::R(d, tl.base + s);
-            tl.r[s] = r;
-            from_zero(F, s, r);
+//
+// It is a chain of ~24 block-wide phases of a few cells each, bound by each phase's latency:
+// two dependent shared-memory reads, eight dependent adds and multiplies and a fast quotient, about
+// 250 cycles. With the way up of the level above: 12.8 -> 7.3 us (32 x 18 cells, 4 levels),
+// 17.9 -> 10.2 us (48 x 27, 6 levels).
+constexpr int kTailJ = 3;   // a first tail level has at most 1500 cells, 750 of a colour
+template <bool SLOW>
+DEV bool tail_cycle(const float2* R, const Tail& tl) {
+    bool bad = false;
+    const int last = tl.nl - 1;
+    TailLevel L = tl.lv[0];
+    {   // (every load in flight before the first is used)
+        constexpr int PER = 6;
+        float2 v[PER];
+#pragma unroll
+        for (int j = 0; j < PER; j++) v[j] = R[min((int)threadIdx.x + j * NT, tl.nf - 1)];
+#pragma unroll
+        for (int j = 0; j < PER; j++) {
+            const int s = threadIdx.x + j * NT;
+            if (s < tl.nf) tail_rhs<SLOW>(tl, s, L.n0, v[j], bad);
         }
     }
     __syncthreads();
-    // a half-sweep: every slot's reads are issued before its terms are summed (neighbour
-    // slots clamped into the level and kept or not by the mask), in the shader's order
-    auto sweep = [&](const Lv& L, int colour) {
-        const int o = L.off - tl.base, n = L.w * L.h;
-        const int lo = o, hi = o + n - 1;
-        for (int t = threadIdx.x; t < n; t += NT) {
-            const int y = qdiv(t, L.wm), x = t - y * L.w;
-            const int s = o + t;
-            const float D = tl.dg[s];
-            const float2 r = tl.r[s];
-            const bool mine = !(D <= 0.0f) && ((x + y) & 1) == colour;
-            const float4 w = tail_a<M>(d, tl, s);
-            const uint32_t m = tl.m[s];
-            const float2 x0 = tl.x[max(s - 1, lo)], x1 = tl.x[min(s + 1, hi)];
-            const float2 x2 = tl.x[max(s - L.w, lo)], x3 = tl.x[min(s + L.w, hi)];
-            float2 sum = r;
-            if (m & 1u) { sum.x += w.x * x0.x; sum.y += w.x * x0.y; }
-            if (m & 2u) { sum.x += w.y * x1.x; sum.y += w.y * x1.y; }
-            if (m & 4u) { sum.x += w.z * x2.x; sum.y += w.z * x2.y; }
-            if (m & 8u) { sum.x += w.w * x3.x; sum.y += w.w * x3.y; }
-            if (mine) tl.x[s] = divz(sum, D);
-        }
-        __syncthreads();
-    };
-    for (int l = first; l < last; l++) {
-        Lv L = lev(d.lv, l), C = lev(d.lv, l + 1);
-        const int o = L.off - tl.base, oc = C.off - tl.base;
-        sweep(L, 1);
-        for (int t = threadIdx.x; t < C.w * C.h; t += NT) {
-            const int ccy = qdiv(t, C.wm), ccx = t - ccy * C.w;
-            float sumx = 0.0f, sumy = 0.0f;
-            const int step[4] = {-1, 1, -L.w, L.w};
-            for (int k = 0; k < 4; k++) {
-                int cx = 2 * ccx + (k & 1), cy = 2 * ccy + (k >> 1);
-                if (!l_inside(L, cx, cy)) continue;
-                int s = o + cy * L.w + cx;
-                const uint32_t m = tl.m[s];
-                if (!(m & 16u)) continue;
-                float4 w = tail_a<M>(d, tl, s);
-                float Ds = tl.dg[s];
-                float2 xs = tl.x[s];
-                float azx = Ds * xs.x, azy = Ds * xs.y;
-                for (int q = 0; q < 4; q++) {
-                    if (m & (1u << q)) {
-                        float wd = wcomp(w, q);
-                        float2 xn = tl.x[s + step[q]];
-                        azx -= wd * xn.x;
-                        azy -= wd * xn.y;
-                    }
-                }
-                float2 rh = tl.r[s];
-                sumx += rh.x - azx;
-                sumy += rh.y - azy;
-            }
-            tl.r[oc + t] = make_float2(sumx, sumy);
-            from_zero(C, t, make_float2(sumx, sumy));
-        }
-        __syncthreads();
+    tail_sweep<SLOW, kTailJ>(tl, L.o + L.n0, L.n1, L.w, bad);
+#pragma unroll 1
+    for (int l = 0; l < last; l++) {
+        const TailLevel C = tl.lv[l + 1];
+        tail_restrict<SLOW>(tl, L, C, bad);
+        L = C;
+        tail_sweep<SLOW, 1>(tl, L.o + L.n0, L.n1, L.w, bad);
     }
-    {
-        Lv L = lev(d.lv, last);
-        for (int s = 1; s < 9; s++) sweep(L, s & 1);
+    // the coarsest level's other seven half-sweeps (it has at most 4 cells, unless it is the first)
+#pragma unroll 1
+    for (int k = 0; k < 7; k++) {
+        const bool odd = k & 1;
+        if (last > 0) tail_sweep<SLOW, 1>(tl, odd ? L.o + L.n0 : L.o, odd ? L.n1 : L.n0, L.w, bad);
+        else tail_sweep<SLOW, kTailJ>(tl, odd ? L.o + L.n0 : L.o, odd ? L.n1 : L.n0, L.w, bad);
     }
-    for (int l = last - 1; l >= first; l--) {
-        Lv F = lev(d.lv, l), C = lev(d.lv, l + 1);
-        const int o = F.off - tl.base, oc = C.off - tl.base;
-        for (int t = threadIdx.x; t < F.w * F.h; t += NT) {
-            const int y = qdiv(t, F.wm), x = t - y * F.w;
-            if (((x + y) & 1) == 0) continue;
-            int s = o + t;
-            float D = tl.dg[s];
-            if (D <= 0.0f) continue;
-            float4 w = tail_a<M>(d, tl, s);
-            float2 sum = tl.r[s];
-            const uint32_t m = tl.m[s];
-            for (int q = 0; q < 4; q++) {
-                int nx = x + NBX[q], ny = y + NBY[q];
-                if (!(m & (1u << q))) continue;
-                float wd = wcomp(w, q);
-                float2 xn = tl.x[o + ny * F.w + nx];
-                float2 xc = tl.x[oc + (ny >> 1) * C.w + (nx >> 1)];
-                sum.x += wd * (xn.x + MG_OMEGA * xc.x);
-                sum.y += wd * (xn.y + MG_OMEGA * xc.y);
-            }
-            tl.x[s] = divz(sum, D);
-        }
-        __syncthreads();
-        sweep(F, 0);
+#pragma unroll 1
+    for (int l = last - 1; l >= 1; l--) {
+        const TailLevel C = L;
+        L = tl.lv[l];
+        tail_correct<SLOW, 1>(tl, L, C, bad);
+        tail_sweep<SLOW, 1>(tl, L.o, L.n0, L.w, bad);
     }
-    if (writer)   // the first tail level's result (for inspection; a batch's way up reads it)
-        for (int s = threadIdx.x; s < tl.nf; s += NT) M::setZ(d, tl.base + s, tl.x[s]);
+    if (last > 0) {
+        const TailLevel C = L;
+        L = tl.lv[0];
+        tail_correct<SLOW, kTailJ>(tl, L, C, bad);
+        tail_sweep<SLOW, kTailJ>(tl, L.o, L.n0, L.w, bad);
+    }
+    return bad;
+}
+// (only where an operand left the fast quotients' range, which may have left NaN in the iterates:
+// a zero coupling does not hide one)
+static __device__ __noinline__ void tail_slow(const float2* R, int T, int nf, int nl) {
+    const Tail tl = tail_at(dyn_smem + kTileBytes, reinterpret_cast<float2*>(dyn_smem), 0, T, nf, nl);
+    for (int s = threadIdx.x; s < T; s += NT) tl.x[s] = make_float2(0.0f, 0.0f);
+    __syncthreads();
+    tail_cycle<true>(R, tl);
+}
+// (Z: where the first tail level's result goes, for inspection; a batch's way up reads it)
+DEV void phase_tail(const float2* R, float2* Z, const Tail& tl) {
+    if (__syncthreads_or(tail_cycle<false>(R, tl))) tail_slow(R, tl.T, tl.nf, tl.nl);
+    if (Z)
+        for (int s = threadIdx.x; s < tl.nf; s += NT) Z[s] = tl.x[s];
 }
 
 // The active-tile lists of levels 0 .. tail - 1 of scene d (one block), from ptile.
@@ -937,76 +1184,76 @@ struct TileCache {
     uint32_t cnt[kCacheLevels];
     uint32_t item[kCacheLevels][kCachePer];
 };
+template <class I>
+DEV void fill_level(TileCache& tc, int l, uint32_t tiles, I&& item) {
+    if (threadIdx.x == 0) tc.cnt[l] = tiles;
+    for (int k = threadIdx.x; k < kCachePer; k += NT) {
+        const uint32_t j = blockIdx.x + (uint32_t)k * gridDim.x;
+        if (j < tiles) tc.item[l][k] = item(j);
+    }
+}
+// how many of a level's tiles this block takes, and the k-th of them
+DEV int my_count(uint32_t tiles) { return blockIdx.x < tiles ? (int)((tiles - blockIdx.x + gridDim.x - 1) / gridDim.x) : 0; }
+template <class I>
+DEV uint32_t my_item(const TileCache& tc, int l, int k, I&& item) {
+    return (l < kCacheLevels && k < kCachePer) ? tc.item[l][k] : item(blockIdx.x + (uint32_t)k * gridDim.x);
+}
+struct EveryOne {
+    DEV int operator()(int k) const { return k; }
+};
 
+DEV uint32_t active_tiles(const DevScene& d, int l, const TileCache& tc) {
+    return l < kCacheLevels ? tc.cnt[l] : *(volatile uint32_t*)&d.pcount[l];
+}
 DEV void fill_cache(const DevScene& d, TileCache& tc) {
     for (int l = 0; l < kCacheLevels && l < d.lv.tail; l++) {
-        const uint32_t cnt = *(volatile uint32_t*)&d.pcount[l];
         const uint32_t* list = d.plist + d.lv.toff[l];
-        if (threadIdx.x == 0) tc.cnt[l] = cnt;
-        for (int k = threadIdx.x; k < kCachePer; k += NT) {
-            const uint32_t j = blockIdx.x + (uint32_t)k * gridDim.x;
-            if (j < cnt) tc.item[l][k] = list[j];
-        }
+        fill_level(tc, l, *(volatile uint32_t*)&d.pcount[l], [&](uint32_t k) { return list[k]; });
     }
     __syncthreads();
 }
-
-// For every active tile of level l of scene d, in this block's share of the list.
-template <class F>
-DEV void for_active(const DevScene& d, int l, const TileCache& tc, F&& f) {
-    const bool cached = l < kCacheLevels;
-    const uint32_t cnt = cached ? tc.cnt[l] : *(volatile uint32_t*)&d.pcount[l];
-    const uint32_t* list = d.plist + d.lv.toff[l];
-    int k = 0;
-    for (uint32_t j = blockIdx.x; j < cnt; j += gridDim.x, k++)
-        f((int)((cached && k < kCachePer) ? tc.item[l][k] : list[j]));
+DEV int my_tile(const DevScene& d, const TileCache& tc, int l, int k) {
+    return (int)my_item(tc, l, k, [&](uint32_t j) { return d.plist[d.lv.toff[l] + j]; });
 }
 
-// The same share through the two-region pipeline (stage / finish halves of a tile body).
-template <class S, class F>
-DEV void pipe_active(const DevScene& d, int l, const TileCache& tc, Region* rg, S&& stage, F&& finish) {
-    const bool cached = l < kCacheLevels;
-    const uint32_t cnt = cached ? tc.cnt[l] : *(volatile uint32_t*)&d.pcount[l];
+// For every active tile of level l of scene d, one at a time by the whole block.
+template <class F>
+DEV void for_active(const DevScene& d, int l, const TileCache& tc, F&& f) {
+    const uint32_t cnt = active_tiles(d, l, tc);
     const uint32_t* list = d.plist + d.lv.toff[l];
-    pipe_tiles(
-        cnt, [&](int k) { return (cached && k < kCachePer) ? tc.item[l][k] : list[blockIdx.x + (uint32_t)k * gridDim.x]; },
-        rg, [&](uint32_t t, Region& r) { stage((int)t, r); }, [&](uint32_t t, Region& r) { finish((int)t, r); });
+    for (uint32_t j = blockIdx.x; j < cnt; j += gridDim.x) f((int)list[j]);
 }
 
 // Whether this block computes the tail of scene d: it owns a tile of the level above the tail
 // (whose way up reads the tail's result from the block's own copy), or it is block 0.
 DEV bool tail_reader(const DevScene& d, const TileCache& tc) {
-    const int l = d.lv.tail - 1;
-    const uint32_t cnt = l < kCacheLevels ? tc.cnt[l] : *(volatile uint32_t*)&d.pcount[l];
-    return blockIdx.x == 0 || blockIdx.x < cnt;
+    return blockIdx.x == 0 || blockIdx.x < active_tiles(d, d.lv.tail - 1, tc);
 }
 
-// One V-cycle of one scene: level 0's right-hand side through R (fused with the CG update
-// when R.q is set), result in mgz of level 0, partials of r.z and r.r. Returns false on a
-// barrier timeout.
+// One V-cycle of one scene: level 0's right-hand side through A (fused with the CG update
+// when A.q is set), result in mgz of level 0, partials of r.z and r.r; r_new: the residual
+// after the update. Returns false on a barrier timeout.
 template <class M>
-DEV bool vcycle(const DevScene& d, const Tail& tl, const Rsrc<M>& R, float2* r_out, const float2* p, const float2* r_new,
-                float2* sz, typename M::acc4* buf, Region* rg, const TileCache& tc) {
+DEV bool vcycle(const DevScene& d, const Geo& g, const Tail& tl, const DownArgs& A, const float2* r_new, const TileCache& tc) {
     const int tail = d.lv.tail;
+    auto of = [&d](int) -> const DevScene& { return d; };
+#pragma unroll 1
     for (int l = 0; l < tail; l++) {
-        Rsrc<M> Rl = R;
-        if (l > 0) Rl = Rsrc<M>{nullptr, nullptr, 0.0f, 0.0f};
-        float2* ro = l == 0 ? r_out : nullptr;
         const Lv F = lev(d.lv, l), C = lev(d.lv, l + 1);
-        pipe_active(d, l, tc, rg, [&](int t, Region& r) { stage_down<M>(d, F, t, Rl, ro != nullptr, p, r); },
-                    [&](int t, Region& r) { finish_down<M>(d, F, C, t, Rl, ro, sz, r); });
+        DownArgs D = A;
+        if (l > 0) D = DownArgs{d.mgr, nullptr, 0.0f, 0.0f, nullptr, nullptr};
+        down_pass<M>(g, my_count(active_tiles(d, l, tc)), l == 0, of, [&](int k) { return DownTile{0, F, C, my_tile(d, tc, l, k), D}; }, EveryOne());
         if (!grid_sync(d.K)) return false;
     }
     // only the blocks with a tile of the level above the tail read the tail's result (from
     // their own copy); block 0 also stores it
-    if (tail_reader(d, tc)) phase_tail<M>(d, tl, blockIdx.x == 0);
+    if (tail_reader(d, tc)) phase_tail(d.mgr + tl.base, blockIdx.x == 0 ? d.mgz + tl.base : nullptr, tl);
+#pragma unroll 1
     for (int l = tail - 1; l >= 0; l--) {
-        const Lv C = lev(d.lv, l + 1);
-        const Zc zc{(l == tail - 1) ? tl.x : nullptr, C.off, C.w};
-        const Rsrc<M> rhs = l == 0 ? Rsrc<M>{r_new, nullptr, 0.0f, 0.0f} : Rsrc<M>{nullptr, nullptr, 0.0f, 0.0f};
-        const Lv F = lev(d.lv, l);
-        pipe_active(d, l, tc, rg, [&](int t, Region& r) { stage_up<M>(d, F, t, rhs, zc, r); },
-                    [&](int t, Region& r) { finish_up<M>(d, F, t, l == 0, zc, sz, buf, r); });
+        const Lv F = lev(d.lv, l), C = lev(d.lv, l + 1);
+        const float2* zs = l == tail - 1 ? tl.x : nullptr;
+        const float2* r = l == 0 ? r_new : d.mgr;
+        up_pass<M>(g, my_count(active_tiles(d, l, tc)), l == 0, of, [&](int k) { return UpTile{0, F, C, my_tile(d, tc, l, k), r, d.mgz + C.off, zs}; }, EveryOne());
         if (!grid_sync(d.K)) return false;
     }
     return true;
@@ -1143,90 +1390,6 @@ DEV bool decide_check(Solve<T>& K, const Dbl4& tot) {
     return adopt;
 }
 
-// cg_apply.comp on level-0 tile t: p = z + beta p_old, q = A p (the FP32 operator), the
-// tile's sum of p.q into part[n + t]. Copies (one ring around the tile is enough): the
-// operator's diagonal, z (u) and p_old (v, unless both betas are zero); the couplings of the
-// tile's own cells.
-DEV void stage_apply(const DevScene& d, const Lv& F, int t, bool nob, const float2* p_old, Region& rg) {
-    const int2 og = tile_origin(F, t);
-    const int ox = og.x, oy = og.y;
-#pragma unroll
-    for (int j = 0; j < RJ; j++) {
-        const int k = threadIdx.x + j * NT;
-        if (k >= RN) break;
-        const int kx = k % RW, ky = k / RW;
-        if (kx == 0 || ky == 0 || kx == RW - 1 || ky == RW - 1) continue;
-        const int x = ox - RH + kx, y = oy - RH + ky;
-        const bool in = l_inside(F, x, y);
-        const int i = in ? l_at(F, x, y) : 0;
-        cp_async<4>(&rg.dg[k], d.mgd + i, in);
-        cp_async<8>(&rg.u[k], d.mgz + i, in);
-        if (!nob) cp_async<8>(&rg.v[k], p_old + i, in);
-    }
-    const int cx = ox + (threadIdx.x & 15), cy = oy + (threadIdx.x >> 4);
-    const bool in = l_inside(F, cx, cy);
-    cp_async<16>(&rg.a[rslot(threadIdx.x & 15, threadIdx.x >> 4)], d.mga + (in ? l_at(F, cx, cy) : 0), in);
-}
-
-template <class M>
-DEV void finish_apply(const DevScene& d, const Lv& F, int t, float b0, float b1, float2* p_new, typename M::acc4* buf,
-                      Region& rg) {
-    using acc = typename M::acc;
-    const int n = d.nwg;
-    typename M::acc4* part = M::part(d) + n;
-    const bool nob = b0 == 0.0f && b1 == 0.0f;
-    const int2 og = tile_origin(F, t);
-    const int ox = og.x, oy = og.y;
-    __syncthreads();   // (every thread's copies have landed)
-    auto dg = [&](int k) {
-        const float v = rg.dg[k];
-        return v > 0.0f ? v : 0.0f;
-    };
-    auto dir = [&](int k) {   // the direction p = z + beta p_old
-        const float2 z = rg.u[k];
-        if (nob) return z;
-        const float2 po = rg.v[k];
-        return make_float2(b0 != 0.0f ? z.x + b0 * po.x : z.x, b1 != 0.0f ? z.y + b1 * po.y : z.y);
-    };
-    const int cx = ox + (threadIdx.x & 15), cy = oy + (threadIdx.x >> 4);
-    const int k0 = rslot(threadIdx.x & 15, threadIdx.x >> 4);
-    typename M::acc4 a4 = M::zero4();
-    if (l_inside(F, cx, cy)) {
-        const int i = l_at(F, cx, cy);
-        const float D = dg(k0);
-        if (D > 0.0f) {
-            const float2 pp = dir(k0);
-            const float4 w = rg.a[k0];
-            float dn[4];
-            float2 pn[4];
-#pragma unroll
-            for (int q = 0; q < 4; q++) {
-                dn[q] = dg(k0 + RSTEP[q]);
-                pn[q] = dir(k0 + RSTEP[q]);
-            }
-            float qx = D * pp.x, qy = D * pp.y;
-#pragma unroll
-            for (int q = 0; q < 4; q++) {
-                const float wd = wcomp(w, q);
-                const float ux = wd * pn[q].x, uy = wd * pn[q].y;
-                if (dn[q] > 0.0f) {
-                    qx -= ux;
-                    qy -= uy;
-                }
-            }
-            p_new[i] = pp;
-            d.cgq[i] = make_float2(qx, qy);
-            a4 = M::prod4(0.0f, 0.0f, 0.0f, 0.0f, pp.x, qx, pp.y, qy);
-        } else {
-            p_new[i] = make_float2(0.0f, 0.0f);
-        }
-    }
-    buf[threadIdx.x] = a4;
-    block_tree(buf);
-    if (threadIdx.x == 0) part[t] = buf[0];
-    __syncthreads();
-}
-
 template <class T>
 DEV T mix_was(T a, T keep, uint32_t was) { return mixf(a, keep, (float)was); }
 template <>
@@ -1334,26 +1497,21 @@ DEV void scal_stats(SolveState* G, const Solve<T>& K, int second, double true_re
 // The whole pressure solve. `second`: the solve after the implicit viscosity (cg_reduce
 // mode 8/9: same matrix and hierarchy, density correction counted as solved).
 template <class M>
-__global__ void __launch_bounds__(NT, 2) k_mgpcg(DevScene d, int second, int scale_mode) {
+__global__ void __launch_bounds__(NT, 2) k_mgpcg(const __grid_constant__ DevScene d, int second, int scale_mode) {
     grid_begin(d.K);
     using acc = typename M::acc;
     using acc4 = typename M::acc4;
     __shared__ TileCache tc;
-    __shared__ float2 sz[NT];
     // the block's tree buffer: float pairs in mixed precision (the refinement's checks), whose
     // bytes the dot products' trees use as acc4 in other phases
     __shared__ typename std::conditional<M::kMixed, FF4, acc4>::type buf_raw[NT];
     acc4* buf = reinterpret_cast<acc4*>(buf_raw);
     __shared__ Solve<acc> K;
-    // dynamic: the staging regions, then the tail levels (matrices, iterates, masks: kept for
-    // the whole solve); the tail's right-hand sides, live only in the tail phase, when no
-    // tile is being staged, in the regions' bytes
-    extern __shared__ __align__(16) unsigned char dyn_smem[];
-    Region* rg = reinterpret_cast<Region*>(dyn_smem);
     const DevParams* P = d.P;
     const int n = d.nwg;
     acc4* part = M::part(d);
-    const Tail tl = make_tail(d, dyn_smem + kDepth * sizeof(Region), reinterpret_cast<float2*>(dyn_smem));
+    const Tail tl = make_tail(d);
+    const Geo g = geo();
     if (!second) {
         for (int t = blockIdx.x; t < n; t += gridDim.x) cg_scale_tile<M>(d, t, scale_mode);
         for (int l = 1; l <= d.lv.tail; l++) {
@@ -1376,53 +1534,49 @@ __global__ void __launch_bounds__(NT, 2) k_mgpcg(DevScene d, int second, int sca
     // b.b now, while nothing writes the second half of the partials: the first apply phase
     // after the V-cycle does, and a block can reach it before a slower one has summed them
     const auto b = M::fin(total(part + n, n, buf));
-    if (!vcycle<M>(d, tl, Rsrc<M>{r_cur, nullptr, 0.0f, 0.0f}, nullptr, nullptr, r_cur, sz, buf, rg, tc)) return;
     const acc tx = (acc)P->tol[0], ty = (acc)P->tol[1];
-    {
-        const auto a = M::fin(total(part, n, buf));
-        if (threadIdx.x == 0) scal_start<acc>(K, a, b, tx, ty, second);
-        __syncthreads();
-    }
     float2* p_old = d.cgp;
     float2* p_new = d.cgp2;
     const Lv L0 = lev(d.lv, 0);
     const uint32_t cap = d.K->cap[second ? 1 : 0];   // this frame's recorded iterations
-    for (uint32_t it = 0; it < cap; it++) {
-        if (K.done[0] && K.done[1]) break;
-        if constexpr (M::kMixed) {
-            // the refinement (the same decisions in every block: the same K); q is free until
-            // the apply phase rewrites it, and the partials' second half until it sums p.q
-            if (it > 0 && want_check(K)) {
-                FF4* pc = reinterpret_cast<FF4*>(d.partials64) + n;
-                for_active(d, 0, tc, [&](int t) { check_tile(d, t, d.cgq, pc, reinterpret_cast<FF4*>(buf_raw)); });
-                if (!grid_sync(d.K)) return;
-                const Dbl4 tot = to_dbl(total(pc, n, reinterpret_cast<FF4*>(buf_raw)));
-                __shared__ int s_adopt;
-                if (threadIdx.x == 0) s_adopt = decide_check(K, tot) ? 1 : 0;
-                __syncthreads();
-                if (s_adopt) {
-                    for_active(d, 0, tc, [&](int t) { adopt_tile(d, t, d.cgq, r_cur); });
+    // it = 0: the start (a V-cycle on the residual of x0); it > 0: the iterations
+    for (uint32_t it = 0;; it++) {
+        DownArgs A{r_cur, nullptr, 0.0f, 0.0f, nullptr, nullptr};
+        if (it > 0) {
+            if (it > cap || (K.done[0] && K.done[1])) break;
+            if constexpr (M::kMixed) {
+                // the refinement (the same decisions in every block: the same K); q is free until
+                // the apply phase rewrites it, and the partials' second half until it sums p.q
+                if (it > 1 && want_check(K)) {
+                    FF4* pc = reinterpret_cast<FF4*>(d.partials64) + n;
+                    for_active(d, 0, tc, [&](int t) { check_tile(d, t, d.cgq, pc, reinterpret_cast<FF4*>(buf_raw)); });
                     if (!grid_sync(d.K)) return;
+                    const Dbl4 tot = to_dbl(total(pc, n, reinterpret_cast<FF4*>(buf_raw)));
+                    __shared__ int s_adopt;
+                    if (threadIdx.x == 0) s_adopt = decide_check(K, tot) ? 1 : 0;
+                    __syncthreads();
+                    if (s_adopt) {
+                        for_active(d, 0, tc, [&](int t) { adopt_tile(d, t, d.cgq, r_cur); });
+                        if (!grid_sync(d.K)) return;
+                    }
                 }
             }
-        }
-        const float b0 = (float)K.beta[0], b1 = (float)K.beta[1];
-        const bool nob = b0 == 0.0f && b1 == 0.0f;
-        pipe_active(d, 0, tc, rg, [&](int t, Region& r) { stage_apply(d, L0, t, nob, p_old, r); },
-                    [&](int t, Region& r) { finish_apply<M>(d, L0, t, b0, b1, p_new, buf, r); });
-        if (!grid_sync(d.K)) return;
-        {
-            const auto b = M::fin(total(part + n, n, buf));
-            if (threadIdx.x == 0) scal_alpha<acc>(K, b);
+            const float b0 = (float)K.beta[0], b1 = (float)K.beta[1];
+            apply_pass<M>(my_count(active_tiles(d, 0, tc)), [&d](int) -> const DevScene& { return d; }, [&](int k) { return ApplyTile{0, L0, my_tile(d, tc, 0, k), b0, b1, p_old, p_new}; }, EveryOne());
+            if (!grid_sync(d.K)) return;
+            const auto pq = M::fin(total(part + n, n, buf));
+            if (threadIdx.x == 0) scal_alpha<acc>(K, pq);
             __syncthreads();
+            A = DownArgs{r_cur, d.cgq, (float)K.alpha[0], (float)K.alpha[1], p_new, r_nxt};
         }
-        Rsrc<M> R{r_cur, d.cgq, (float)K.alpha[0], (float)K.alpha[1]};
-        if (!vcycle<M>(d, tl, R, r_nxt, p_new, r_nxt, sz, buf, rg, tc)) return;
-        {
-            const auto a = M::fin(total(part, n, buf));
-            if (threadIdx.x == 0) scal_beta<acc>(K, a, tx, ty);
-            __syncthreads();
+        if (!vcycle<M>(d, g, tl, A, it > 0 ? r_nxt : r_cur, tc)) return;
+        const auto a = M::fin(total(part, n, buf));
+        if (threadIdx.x == 0) {
+            if (it == 0) scal_start<acc>(K, a, b, tx, ty, second);
+            else scal_beta<acc>(K, a, tx, ty);
         }
+        __syncthreads();
+        if (it == 0) continue;
         float2* t = p_old;
         p_old = p_new;
         p_new = t;
@@ -1488,49 +1642,23 @@ DEV uint32_t batch_item(const BatchView& B, int l, int g) {
     return ((uint32_t)s << 16) | d.plist[d.lv.toff[l] + (g - o[s])];
 }
 
+DEV uint32_t active_tiles_b(const BatchView& B, int l, const TileCache& tc) {
+    return l < kCacheLevels ? tc.cnt[l] : *(volatile const uint32_t*)&B.aoff[l * (B.ns + 1) + B.ns];
+}
 DEV void fill_cache_b(const BatchView& B, TileCache& tc) {
-    for (int l = 0; l < kCacheLevels && l < B.max_tail; l++) {
-        const int N = *(volatile const int*)&B.aoff[l * (B.ns + 1) + B.ns];
-        if (threadIdx.x == 0) tc.cnt[l] = (uint32_t)N;
-        for (int k = threadIdx.x; k < kCachePer; k += NT) {
-            const int g = blockIdx.x + k * gridDim.x;
-            if (g < N) tc.item[l][k] = batch_item(B, l, g);
-        }
-    }
+    for (int l = 0; l < kCacheLevels && l < B.max_tail; l++)
+        fill_level(tc, l, *(volatile const uint32_t*)&B.aoff[l * (B.ns + 1) + B.ns], [&](uint32_t k) { return batch_item(B, l, (int)k); });
     __syncthreads();
 }
 
 template <class F>
 DEV void for_active_b(const BatchView& B, int l, const TileCache& tc, F&& f) {
-    const bool cached = l < kCacheLevels;
-    const int N = cached ? (int)tc.cnt[l] : *(volatile const int*)&B.aoff[l * (B.ns + 1) + B.ns];
-    int k = 0;
-    for (int g = blockIdx.x; g < N; g += gridDim.x, k++) {
-        const uint32_t it = (cached && k < kCachePer) ? tc.item[l][k] : batch_item(B, l, g);
+    const uint32_t N = active_tiles_b(B, l, tc);
+    for (uint32_t g = blockIdx.x; g < N; g += gridDim.x) {
+        const uint32_t it = batch_item(B, l, (int)g);
         const int s = (int)(it >> 16);
         f(s, B.scenes[s], (int)(it & 0xffffu));
     }
-}
-
-// The same through the two-region pipeline: stage(s, d, t, rg) / finish(s, d, t, rg).
-template <class S, class F>
-DEV void pipe_active_b(const BatchView& B, int l, const TileCache& tc, Region* rg, S&& stage, F&& finish) {
-    const bool cached = l < kCacheLevels;
-    const int N = cached ? (int)tc.cnt[l] : *(volatile const int*)&B.aoff[l * (B.ns + 1) + B.ns];
-    pipe_tiles(
-        (uint32_t)N,
-        [&](int k) {
-            return (cached && k < kCachePer) ? tc.item[l][k] : batch_item(B, l, (int)(blockIdx.x + (uint32_t)k * gridDim.x));
-        },
-        rg,
-        [&](uint32_t it, Region& r) {
-            const int s = (int)(it >> 16);
-            stage(s, B.scenes[s], (int)(it & 0xffffu), r);
-        },
-        [&](uint32_t it, Region& r) {
-            const int s = (int)(it >> 16);
-            finish(s, B.scenes[s], (int)(it & 0xffffu), r);
-        });
 }
 
 DEV float2* parity_r(const DevScene& d, int it) { return (it & 1) ? d.mgr2 : d.mgr; }
@@ -1538,30 +1666,21 @@ DEV float2* parity_p(const DevScene& d, int it) { return (it & 1) ? d.cgp2 : d.c
 
 }  // namespace
 
-static_assert(sizeof(Region) % 16 == 0, "regions laid end to end in dynamic shared memory");
-
-// The batched solve's dynamic shared memory: the staging regions and, during the tail phase
-// only, one scene's tail (a scene's tail is rebuilt and solved within that phase and its
-// result stored to global memory, while no tile is being staged), in the same bytes.
-size_t pressure_batch_smem(const Levels& lv) {
-    return std::max(tail_bytes(tail_cells(lv), true, tail_first_cells(lv)), (size_t)kDepth * sizeof(Region));
+size_t pressure_smem(const Levels& lv) {
+    return kTileBytes + tail_bytes(tail_cells(lv));
 }
 
 template <class M>
-__global__ void __launch_bounds__(NT, 4) k_mgpcg_batch(BatchView B, int second) {
+__global__ void __launch_bounds__(NT, 2) k_mgpcg_batch(BatchView B, int second) {
     grid_begin(B.K);
     using acc = typename M::acc;
     using acc4 = typename M::acc4;
     __shared__ TileCache tc;
-    __shared__ float2 sz[NT];
     // the block's tree buffer: float pairs in mixed precision (the refinement's checks), whose
     // bytes the dot products' trees use as acc4 in other phases
     __shared__ typename std::conditional<M::kMixed, FF4, acc4>::type buf_raw[NT];
     acc4* buf = reinterpret_cast<acc4*>(buf_raw);
     __shared__ int s_run;
-    extern __shared__ __align__(16) unsigned char dyn_smem[];
-    Region* rg = reinterpret_cast<Region*>(dyn_smem);
-    unsigned char* tail_smem = dyn_smem;
     Solve<acc>* KS = reinterpret_cast<Solve<acc>*>(B.scal);
     SolveState* BK = B.K;
     auto tol = [&](const DevScene& d, int c) { return (acc)d.P->tol[c]; };
@@ -1610,59 +1729,59 @@ __global__ void __launch_bounds__(NT, 4) k_mgpcg_batch(BatchView B, int second) 
         }
         __syncthreads();
     }
+    // one tail per block stays in its shared memory for the whole solve; with more scenes than
+    // blocks, each tail phase sets its tail up again
+    const bool resident = B.ns <= (int)gridDim.x;
+    if (resident && (int)blockIdx.x < B.ns) tail_setup<M>(B.scenes[blockIdx.x], make_tail(B.scenes[blockIdx.x]), false);
+    const Geo geom = geo();
+    auto of = [&B](int s) -> const DevScene& { return B.scenes[s]; };
+    auto item = [&](int l, int k) { return my_item(tc, l, k, [&](uint32_t g) { return batch_item(B, l, (int)g); }); };
     // One V-cycle on every running scene; it < 0: the start (right-hand side the residual
     // of x0, no update); else the iteration's, fused with its update.
     auto vcycle_all = [&](int it) -> bool {
         const bool fused = it >= 0;
         const int ir = fused ? it : 0;
-        for (int l = 0; l < B.max_tail; l++) {
-            auto rsrc = [&](int s, const DevScene& d) {
-                const Solve<acc>& K = KS[s];
-                Rsrc<M> R{nullptr, nullptr, 0.0f, 0.0f};
-                if (l == 0) R = fused ? Rsrc<M>{parity_r(d, ir), d.cgq, (float)K.alpha[0], (float)K.alpha[1]}
-                                      : Rsrc<M>{parity_r(d, ir), nullptr, 0.0f, 0.0f};
-                return R;
+        // the next of this block's items of level l, from its k-th on, whose scene takes part
+        auto live = [&](int l, int count) {
+            return [&, l, count](int k) {
+                while (k < count && fused && !running((int)(item(l, k) >> 16), it)) k++;
+                return k;
             };
-            pipe_active_b(
-                B, l, tc, rg,
-                [&](int s, const DevScene& d, int t, Region& r) {
-                    if (l >= d.lv.tail || (fused && !running(s, it))) return;
-                    stage_down<M>(d, lev(d.lv, l), t, rsrc(s, d), l == 0 && fused, parity_p(d, ir + 1), r);
-                },
-                [&](int s, const DevScene& d, int t, Region& r) {
-                    if (l >= d.lv.tail || (fused && !running(s, it))) return;
-                    finish_down<M>(d, lev(d.lv, l), lev(d.lv, l + 1), t, rsrc(s, d), (l == 0 && fused) ? parity_r(d, ir + 1) : nullptr,
-                                   sz, r);
-                });
+        };
+#pragma unroll 1
+        for (int l = 0; l < B.max_tail; l++) {
+            const int count = my_count(active_tiles_b(B, l, tc));
+            down_pass<M>(geom, count, l == 0, of, [&](int k) {
+                const uint32_t g = item(l, k);
+                const int s = (int)(g >> 16);
+                const DevScene& d = B.scenes[s];
+                DownArgs A{d.mgr, nullptr, 0.0f, 0.0f, nullptr, nullptr};
+                if (l == 0) {
+                    A.r = parity_r(d, ir);
+                    if (fused) A = DownArgs{A.r, d.cgq, (float)KS[s].alpha[0], (float)KS[s].alpha[1], parity_p(d, ir + 1), parity_r(d, ir + 1)};
+                }
+                return DownTile{s, lev(d.lv, l), lev(d.lv, l + 1), (int)(g & 0xffffu), A};
+            }, live(l, count));
             if (!grid_sync(BK)) return false;
         }
         for (int s = blockIdx.x; s < B.ns; s += gridDim.x) {
             if (fused && !running(s, it)) continue;
             const DevScene& d = B.scenes[s];
-            const Tail tl = make_tail(d, tail_smem, nullptr, true);
-            tail_setup<M>(d, tl, false);
-            phase_tail<M>(d, tl, true);
+            const Tail tl = make_tail(d);
+            if (!resident) tail_setup<M>(d, tl, false);
+            phase_tail(d.mgr + tl.base, d.mgz + tl.base, tl);
+            __syncthreads();
         }
         if (!grid_sync(BK)) return false;
+#pragma unroll 1
         for (int l = B.max_tail - 1; l >= 0; l--) {
-            auto zc_of = [&](const DevScene& d) {
+            const int count = my_count(active_tiles_b(B, l, tc));
+            up_pass<M>(geom, count, l == 0, of, [&](int k) {
+                const uint32_t g = item(l, k);
+                const DevScene& d = B.scenes[g >> 16];
                 const Lv C = lev(d.lv, l + 1);
-                return Zc{nullptr, C.off, C.w};
-            };
-            auto rhs_of = [&](const DevScene& d) {
-                return l == 0 ? Rsrc<M>{parity_r(d, fused ? ir + 1 : 0), nullptr, 0.0f, 0.0f}
-                              : Rsrc<M>{nullptr, nullptr, 0.0f, 0.0f};
-            };
-            pipe_active_b(
-                B, l, tc, rg,
-                [&](int s, const DevScene& d, int t, Region& r) {
-                    if (l >= d.lv.tail || (fused && !running(s, it))) return;
-                    stage_up<M>(d, lev(d.lv, l), t, rhs_of(d), zc_of(d), r);
-                },
-                [&](int s, const DevScene& d, int t, Region& r) {
-                    if (l >= d.lv.tail || (fused && !running(s, it))) return;
-                    finish_up<M>(d, lev(d.lv, l), t, l == 0, zc_of(d), sz, buf, r);
-                });
+                return UpTile{(int)(g >> 16), lev(d.lv, l), C, (int)(g & 0xffffu), l == 0 ? parity_r(d, fused ? ir + 1 : 0) : d.mgr, d.mgz + C.off, nullptr};
+            }, live(l, count));
             if (!grid_sync(BK)) return false;
         }
         return true;
@@ -1730,17 +1849,18 @@ __global__ void __launch_bounds__(NT, 4) k_mgpcg_batch(BatchView B, int second) 
                 }
             }
         }
-        pipe_active_b(
-            B, 0, tc, rg,
-            [&](int s, const DevScene& d, int t, Region& r) {
-                if (!running(s, it)) return;
-                const float b0 = (float)KS[s].beta[0], b1 = (float)KS[s].beta[1];
-                stage_apply(d, lev(d.lv, 0), t, b0 == 0.0f && b1 == 0.0f, parity_p(d, it), r);
-            },
-            [&](int s, const DevScene& d, int t, Region& r) {
-                if (!running(s, it)) return;
-                finish_apply<M>(d, lev(d.lv, 0), t, (float)KS[s].beta[0], (float)KS[s].beta[1], parity_p(d, it + 1), buf, r);
+        {
+            const int count = my_count(active_tiles_b(B, 0, tc));
+            apply_pass<M>(count, of, [&](int k) {
+                const uint32_t g = item(0, k);
+                const int s = (int)(g >> 16);
+                const DevScene& d = B.scenes[s];
+                return ApplyTile{s, lev(d.lv, 0), (int)(g & 0xffffu), (float)KS[s].beta[0], (float)KS[s].beta[1], parity_p(d, it), parity_p(d, it + 1)};
+            }, [&](int k) {
+                while (k < count && !running((int)(item(0, k) >> 16), it)) k++;
+                return k;
             });
+        }
         if (!grid_sync(BK)) return;
         for (int s = blockIdx.x; s < B.ns; s += gridDim.x) {
             if (!running(s, it)) continue;
@@ -1777,13 +1897,6 @@ __global__ void __launch_bounds__(NT, 4) k_mgpcg_batch(BatchView B, int second) 
         __syncthreads();
     }
     trace_launch_done(BK);
-}
-
-size_t pressure_smem(const Levels& lv) {
-    // the tail's first level has at most 1500 cells and each coarser level at most half the
-    // one above, so a tail holds fewer than 3000 cells
-    static_assert(kDepth * sizeof(Region) >= 4096 * sizeof(float2), "the tail's right-hand sides fit in the regions");
-    return kDepth * sizeof(Region) + tail_bytes(tail_cells(lv), false);
 }
 
 namespace {
@@ -1938,7 +2051,7 @@ constexpr size_t kStaticBytes =
     align256(kStaticTiles * sizeof(uint32_t)) + align256(kMaxLevels * sizeof(uint32_t)) +   // active-tile lists
     align256(2 * kStaticNwg * sizeof(float4)) +                   // per-tile partial sums
     align256(kStaticTotal * sizeof(float4)) + align256(kStaticTotal * sizeof(float)) +
-    3 * align256(kStaticTotal * sizeof(float2)) + 4 * align256((size_t)kStaticMaxCells * sizeof(float2));
+    4 * align256(kStaticTotal * sizeof(float2)) + 4 * align256((size_t)kStaticMaxCells * sizeof(float2));
 
 static __device__ __align__(256) unsigned char g_solve_scratch[kStaticBytes];
 
@@ -1954,7 +2067,15 @@ __global__ void k_static_prep(DevScene d, const float4* mga, const float* mgd, c
     const int t0 = blockIdx.x * blockDim.x + threadIdx.x;
     for (int i = t0; i < d.lv.total; i += stride) {
         if (i < n0) {
-            d.mga[i] = mga[i];
+            // couplings to cells that are no unknowns count for nothing: zero in the copy, whatever
+            // the caller's hold (the passes rely on their being finite)
+            const int x = i % d.W, y = i / d.W;
+            float4 a = mga[i];
+            if (!(x > 0 && mgd[i - 1] > 0.0f)) a.x = 0.0f;
+            if (!(x + 1 < d.W && mgd[i + 1] > 0.0f)) a.y = 0.0f;
+            if (!(y > 0 && mgd[i - d.W] > 0.0f)) a.z = 0.0f;
+            if (!(y + 1 < d.H && mgd[i + d.W] > 0.0f)) a.w = 0.0f;
+            d.mga[i] = a;
             const float D = mgd[i];
             d.mgd[i] = D;
             float2 b = rhs[i];
@@ -1966,6 +2087,7 @@ __global__ void k_static_prep(DevScene d, const float4* mga, const float* mgd, c
         } else {
             d.mga[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
             d.mgd[i] = 0.0f;
+            d.mgy[i] = make_float2(0.0f, 0.0f);
         }
     }
     const int tw = (d.W + 15) / 16, th = (d.H + 15) / 16;
@@ -2056,6 +2178,7 @@ extern "C" int sprout_pressure_solve_static(uint32_t w, uint32_t h, const float*
     d.partials = reinterpret_cast<float4*>(take(2 * kStaticNwg * sizeof(float4)));
     d.mga = reinterpret_cast<float4*>(take(kStaticTotal * sizeof(float4)));
     d.mgd = reinterpret_cast<float*>(take(kStaticTotal * sizeof(float)));
+    d.mgy = reinterpret_cast<float2*>(take(kStaticTotal * sizeof(float2)));
     d.mgx = reinterpret_cast<float2*>(take(kStaticTotal * sizeof(float2)));
     d.mgz = reinterpret_cast<float2*>(take(kStaticTotal * sizeof(float2)));
     d.mgr = reinterpret_cast<float2*>(take(kStaticTotal * sizeof(float2)));

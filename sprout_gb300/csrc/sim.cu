@@ -275,13 +275,15 @@ struct SproutSim {
         A(d.ledger, 8);
         A(d.mga, (size_t)d.lv.total);
         A(d.mgd, (size_t)d.lv.total);
+        A(d.mgy, (size_t)d.lv.total);
         A(d.mgx, (size_t)d.lv.total);
         A(d.mgz, (size_t)d.lv.total);
         A(d.mgr, (size_t)d.lv.total);
-        A(d.mgr2, nc);
-        A(d.cgp, nc);
-        A(d.cgp2, nc);
-        A(d.cgq, nc);
+        // (one entry more: the level passes read cells in pairs)
+        A(d.mgr2, nc + 1);
+        A(d.cgp, nc + 1);
+        A(d.cgp2, nc + 1);
+        A(d.cgq, nc + 1);
         A(d.ptile, (size_t)d.lv.tiles);
         A(d.plist, (size_t)d.lv.tiles);
         A(d.pcount, (size_t)kMaxLevels);
@@ -1736,7 +1738,7 @@ struct SproutBatch {
             const LaunchCfg& c = sim->cfg;
             scale[k] = (c.visc_mode == 2 && c.twice && c.viscous_warm) ? 1 : 0;
             max_tail = std::max(max_tail, sim->d.lv.tail);
-            smem = std::max(smem, pressure_batch_smem(sim->d.lv));
+            smem = std::max(smem, pressure_smem(sim->d.lv));
         }
         for (int l = 0; l < kMaxLevels; l++) {
             int* o = &off[(size_t)l * (ns + 1)];

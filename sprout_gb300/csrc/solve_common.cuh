@@ -48,6 +48,60 @@ DEV float divp(float a, float b) {
     return divz(a, b);
 }
 
+// a / D from D's staged reciprocal y = RN(1 / D), correctly rounded: one correction of q0 =
+// RN(a y) by its exact remainder (P. Markstein, "Computation of elementary functions on the
+// IBM RISC System/6000 processor", IBM J. Res. Dev. 34, 1990). RN(a y) is within 1.5 ulp of
+// a / D, so the corrected value is off by less than 2^-22 ulp before its one rounding and only
+// quotients that close to a rounding boundary could differ from the IEEE division: all
+// significand pairs whose quotient lies within 2^-19 ulp of one (7.4e8 of them) were compared
+// with it on the CPU, none differed. The remainder is taken as q0 D - a, which keeps the sign
+// of a zero numerator. Holds while nothing leaves the normal range: for a zero, or within
+// [2^-85, 2^85], and D within [2^-40, 2^40], outside which recip() gives NaN.
+DEV float quot_fast(float a, float D, float y) {
+    const float q0 = a * y;
+    const float e = fmaf(q0, D, -a);
+    return fmaf(-e, y, q0);
+}
+DEV bool quot_ok(float a) {
+    const float v = fabsf(a);
+    return (v >= 0x1p-80f && v <= 0x1p80f) || v == 0.0f;
+}
+// the reciprocal quot_fast wants of a positive D (0 for one that is not positive)
+DEV float recip(float D) {
+    if (!(D > 0.0f)) return 0.0f;
+    return D >= 0x1p-40f && D <= 0x1p40f ? 1.0f / D : __int_as_float(0x7fffffff);
+}
+// ... and of a matrix row's: also NaN where a coupling lies outside [2^-25, 2^25] (and is not
+// zero), so that products of couplings and values within [2^-60, 2^60] may be divided fast
+DEV bool coupling_ok(float w) {
+    const float v = fabsf(w);
+    return (v >= 0x1p-25f && v <= 0x1p25f) || v == 0.0f;
+}
+DEV bool value_ok(float a) {
+    const float v = fabsf(a);
+    return (v >= 0x1p-60f && v <= 0x1p60f) || v == 0.0f;
+}
+DEV float recip_row(float D, float4 a) {
+    const float y = recip(D);
+    if (!(D > 0.0f)) return y;
+    return coupling_ok(a.x) && coupling_ok(a.y) && coupling_ok(a.z) && coupling_ok(a.w) ? y : __int_as_float(0x7fffffff);
+}
+// Both columns' a / D for dy = (D, recip(D)), D > 0. The fast form notes operands outside its
+// range in `bad` and the caller then runs the same code once more with SLOW, the IEEE division:
+// a division at every use, inlined or called, was most of the persistent kernels' code, which
+// then missed the instruction cache in every phase. A diagonal that is not positive leaves
+// its (zero) numerator as it is.
+template <bool SLOW>
+DEV float quot1(float a, float2 dy) {
+    if (SLOW) return dy.x > 0.0f ? divz(a, dy.x) : a;
+    return quot_fast(a, dy.x, dy.y);
+}
+template <bool SLOW>
+DEV float2 quot2(float2 a, float2 dy, bool& bad) {
+    if (!SLOW) bad |= !(quot_ok(a.x) && quot_ok(a.y) && dy.y > 0.0f);
+    return make_float2(quot1<SLOW>(a.x, dy), quot1<SLOW>(a.y, dy));
+}
+
 DEV unsigned long long global_ns() {
     unsigned long long t;
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
@@ -253,9 +307,10 @@ DEV void block_tree(T* buf) {
 // total() of reduce_tail.glsl:28-41: thread t sums partials t, t + 256, ... in order,
 // then the tree. Every block calls it and gets the same value.
 template <class T>
-DEV T total(const T* part, int n, T* buf) {
+static __device__ __noinline__ T total(const T* part, int n, T* buf) {
     const int t = threadIdx.x;
     T s{};
+#pragma unroll 4
     for (int k = t; k < n; k += NT) s = add4(s, part[k]);
     buf[t] = s;
     block_tree(buf);
