@@ -316,9 +316,10 @@ DEV int level_tiles(const DevScene& d, int l) {
 // The tail levels' state in each block's shared memory (dynamic, FP32 in both precisions). A
 // level's unknowns are listed by colour, the even cells first: entry p of the list holds the
 // cell's row (couplings, zero towards cells that are no unknowns; diagonal and reciprocal), its
-// slot and its right-hand side, so that a half-sweep's thread finds all of these from its own
-// number alone; the iterates lie by slot (the cells' offsets from the first tail level, the slots
-// of mg_tail.comp), where neighbours are at fixed distances. Slots that are no unknown hold zero.
+// slot, its right-hand side and the entries of its four cells of the level above, so that a
+// thread finds all of these from its own number alone; the iterates lie by slot (the cells'
+// offsets from the first tail level, the slots of mg_tail.comp), where neighbours are at fixed
+// distances. Slots that are no unknown hold zero.
 struct TailLevel {
     int o, n, w, h;     // its cells are slots o .. o + n - 1
     uint32_t wm;        // division constant of the width
@@ -333,7 +334,7 @@ struct Tail {
     float2* r;
     TailLevel* lv;
     uint16_t* slot;  // an entry's slot
-    uint16_t* ent;   // a slot's entry (kNoEntry: no unknown)
+    uint16_t* kid;   // of a coarser level's entry p: the four entries at 4 (p - nf) (kNoEntry: no unknown)
     int base, T, nf, nl;
 };
 
@@ -353,7 +354,7 @@ DEV Tail tail_at(unsigned char* smem, float2* r, int base, int T, int nf, int nl
     tl.x = tl.dy + T;
     tl.r = r;
     tl.slot = reinterpret_cast<uint16_t*>(tl.x + T);
-    tl.ent = tl.slot + T;
+    tl.kid = tl.slot + T;
     return tl;
 }
 
@@ -378,8 +379,9 @@ DEV Tail make_tail(const DevScene& d) {
 
 // Cells of the tail levels, and the tail's bytes without its right-hand sides.
 __host__ __device__ inline int tail_cells(const Levels& lv) { return lv.off[lv.n - 1] + lv.w[lv.n - 1] * lv.h[lv.n - 1] - lv.off[lv.tail]; }
-__host__ __device__ inline size_t tail_bytes(int T) {
-    return (kTailLevels * sizeof(TailLevel) + (size_t)T * (sizeof(float4) + 2 * sizeof(float2) + 2 * sizeof(uint16_t)) + 15) / 16 * 16;
+__host__ __device__ inline size_t tail_bytes(int T, int nf) {
+    return (kTailLevels * sizeof(TailLevel) + (size_t)T * (sizeof(float4) + 2 * sizeof(float2) + sizeof(uint16_t)) +
+            (size_t)(T - nf) * 4 * sizeof(uint16_t) + 15) / 16 * 16;
 }
 
 // mg_tail.comp mode 1 in every block's shared memory, once per solve: the first tail
@@ -427,7 +429,9 @@ DEV void tail_setup(const DevScene& d, const Tail& tl, bool writer) {
         __syncthreads();
     }
     // the lists (an entry's place among its colour does not matter to a half-sweep): the couplings
-    // and diagonals so far lie by slot, so they move through registers, level by level
+    // and diagonals so far lie by slot, so they move through registers, level by level; ent: a
+    // slot's entry, kept where the right-hand sides will be
+    uint16_t* const ent = reinterpret_cast<uint16_t*>(tl.r);
     for (int l = 0; l < tl.nl; l++) {
         const Lv L = lev(d.lv, d.lv.tail + l);
         TailLevel& Q = tl.lv[l];
@@ -456,11 +460,20 @@ DEV void tail_setup(const DevScene& d, const Tail& tl, bool writer) {
             if (t >= Q.n) break;
             int e = p[j];
             if (e >= Q.n0) e -= gap;
-            tl.ent[Q.o + t] = e < 0 ? (uint16_t)kNoEntry : (uint16_t)(Q.o + e);
+            ent[Q.o + t] = e < 0 ? (uint16_t)kNoEntry : (uint16_t)(Q.o + e);
             if (e < 0) continue;
             tl.a[Q.o + e] = a[j];
             tl.dy[Q.o + e] = dy[j];
             tl.slot[Q.o + e] = (uint16_t)(Q.o + t);
+        }
+    }
+    __syncthreads();
+    for (int l = 1; l < tl.nl; l++) {
+        const TailLevel F = tl.lv[l - 1], C = tl.lv[l];
+        for (int t = threadIdx.x; t < 4 * (C.n0 + C.n1); t += NT) {
+            const int p = C.o + (t >> 2), c = tl.slot[p] - C.o, cy = qdiv(c, C.wm), cx = c - cy * C.w;
+            const int x = 2 * cx + (t & 1), y = 2 * cy + ((t >> 1) & 1);
+            tl.kid[4 * (p - tl.nf) + (t & 3)] = x < F.w && y < F.h ? ent[F.o + y * F.w + x] : (uint16_t)kNoEntry;
         }
     }
     __syncthreads();
@@ -1035,51 +1048,45 @@ DEV void tail_correct(const Tail& tl, const TailLevel& L, const TailLevel& C, bo
     }
     __syncthreads();
 }
-// The right-hand side of slot s of a tail level, and its first half-sweep, which starts from
+// The right-hand side of entry p of a tail level, and its first half-sweep, which starts from
 // zero: the level's even unknowns (entries below odd) are r / D. The odd ones are written before
 // anything reads them.
 template <bool SLOW>
-DEV void tail_rhs(const Tail& tl, int s, int odd, float2 r, bool& bad) {
-    const uint32_t p = tl.ent[s];
-    if (p == kNoEntry) return;
-    tl.r[p] = r;
-    if ((int)p < odd) tl.x[s] = quot2<SLOW>(r, tl.dy[p], bad);
+DEV void tail_rhs(const Tail& tl, int p, int s, int odd, float2 dy, float2 r, bool on, bool& bad) {
+    const float2 x = quot2<SLOW>(r, dy, bad);
+    if (on) tl.r[p] = r;
+    if (on && p < odd) tl.x[s] = x;
 }
-// The residual of level L summed over the 2 x 2 cells of each cell of level C, four lanes to a
-// coarse cell, one per fine cell: a cell that is no unknown adds nothing (the sum is never -0,
-// so leaving it out or adding +0 is the same).
+// The residual of the level above summed over the four cells of each entry of level C (w: the
+// width above), four lanes to an entry, one per cell: a cell that is no unknown adds nothing (the
+// sum is never -0, so leaving it out or adding +0 is the same).
 template <bool SLOW>
-DEV void tail_restrict(const Tail& tl, const TailLevel& L, const TailLevel& C, bool& bad) {
-    const int cnt = 4 * C.n, k = threadIdx.x & 3, b = threadIdx.x & 28;
+DEV void tail_restrict(const Tail& tl, const TailLevel& C, int w, bool& bad) {
+    const int cnt = 4 * (C.n0 + C.n1), b = threadIdx.x & 28;
 #pragma unroll 1
     for (int t = threadIdx.x; (t & ~31) < cnt; t += NT) {
-        const int c = min(t >> 2, C.n - 1), cy = qdiv(c, C.wm), cx = c - cy * C.w;
-        const int x = 2 * cx + (k & 1), y = 2 * cy + (k >> 1);
-        const bool in = x < L.w && y < L.h;
-        const int s = in ? L.o + y * L.w + x : L.o;
-        const uint32_t p = tl.ent[s];
-        const bool on = in && p != kNoEntry;
-        float2 e = make_float2(0.0f, 0.0f);
-        if (on) {
-            const float4 a = tl.a[p];
-            const float2 rh = tl.r[p], xs = tl.x[s];
-            const float D = tl.dy[p].x;
-            const float2 x0 = tl.x[max(s - 1, 0)], x1 = tl.x[min(s + 1, tl.T - 1)];
-            const float2 x2 = tl.x[max(s - L.w, 0)], x3 = tl.x[min(s + L.w, tl.T - 1)];
-            float2 z = make_float2(D * xs.x, D * xs.y);
-            z.x -= a.x * x0.x; z.y -= a.x * x0.y;
-            z.x -= a.y * x1.x; z.y -= a.y * x1.y;
-            z.x -= a.z * x2.x; z.y -= a.z * x2.y;
-            z.x -= a.w * x3.x; z.y -= a.w * x3.y;
-            e = make_float2(rh.x - z.x, rh.y - z.y);
-        }
+        const int u = min(t, cnt - 4 + (t & 3)), p = C.o + (u >> 2);
+        const uint32_t q = tl.kid[4 * (C.o - tl.nf) + u];
+        const bool on = q != kNoEntry;
+        const int e = on ? (int)q : 0, s = tl.slot[e], cs = tl.slot[p];
+        const float4 a = tl.a[e];
+        const float2 rh = tl.r[e], cdy = tl.dy[p];
+        const float D = tl.dy[e].x;
+        const float2 xs = tl.x[s], x0 = tl.x[max(s - 1, 0)], x1 = tl.x[min(s + 1, tl.T - 1)];
+        const float2 x2 = tl.x[max(s - w, 0)], x3 = tl.x[min(s + w, tl.T - 1)];
+        float2 z = make_float2(D * xs.x, D * xs.y);
+        z.x -= a.x * x0.x; z.y -= a.x * x0.y;
+        z.x -= a.y * x1.x; z.y -= a.y * x1.y;
+        z.x -= a.z * x2.x; z.y -= a.z * x2.y;
+        z.x -= a.w * x3.x; z.y -= a.w * x3.y;
+        const float ex = on ? rh.x - z.x : 0.0f, ey = on ? rh.y - z.y : 0.0f;
         float2 v = make_float2(0.0f, 0.0f);
 #pragma unroll
-        for (int q = 0; q < 4; q++) {
-            v.x += __shfl_sync(0xffffffffu, e.x, b + q);
-            v.y += __shfl_sync(0xffffffffu, e.y, b + q);
+        for (int k = 0; k < 4; k++) {
+            v.x += __shfl_sync(0xffffffffu, ex, b + k);
+            v.y += __shfl_sync(0xffffffffu, ey, b + k);
         }
-        if (k == 0 && t < cnt) tail_rhs<SLOW>(tl, C.o + c, C.o + C.n0, v, bad);
+        tail_rhs<SLOW>(tl, p, cs, C.o + C.n0, cdy, v, (t & 3) == 0 && t < cnt, bad);
     }
     __syncthreads();
 }
@@ -1101,43 +1108,47 @@ DEV bool tail_cycle(const float2* R, const Tail& tl) {
     TailLevel L = tl.lv[0];
     {   // (every load in flight before the first is used)
         constexpr int PER = 6;
+        const int cnt = L.n0 + L.n1;
+        int s[PER];
         float2 v[PER];
 #pragma unroll
-        for (int j = 0; j < PER; j++) v[j] = R[min((int)threadIdx.x + j * NT, tl.nf - 1)];
+        for (int j = 0; j < PER; j++) {
+            if ((int)(threadIdx.x & ~31u) + j * NT >= cnt) break;
+            s[j] = tl.slot[min((int)threadIdx.x + j * NT, cnt - 1)];
+            v[j] = R[s[j]];
+        }
 #pragma unroll
         for (int j = 0; j < PER; j++) {
-            const int s = threadIdx.x + j * NT;
-            if (s < tl.nf) tail_rhs<SLOW>(tl, s, L.n0, v[j], bad);
+            if ((int)(threadIdx.x & ~31u) + j * NT >= cnt) break;
+            const int p = min((int)threadIdx.x + j * NT, cnt - 1);
+            tail_rhs<SLOW>(tl, p, s[j], L.n0, tl.dy[p], v[j], true, bad);
         }
     }
     __syncthreads();
-    tail_sweep<SLOW, kTailJ>(tl, L.o + L.n0, L.n1, L.w, bad);
+    // a level's cells of one colour are one a thread unless there are more than a block's threads
+    auto sweep = [&](bool odd) {
+        const int cnt = odd ? L.n1 : L.n0, p0 = odd ? L.o + L.n0 : L.o;
+        if (cnt <= NT) tail_sweep<SLOW, 1>(tl, p0, cnt, L.w, bad);
+        else tail_sweep<SLOW, kTailJ>(tl, p0, cnt, L.w, bad);
+    };
+    sweep(true);
 #pragma unroll 1
     for (int l = 0; l < last; l++) {
         const TailLevel C = tl.lv[l + 1];
-        tail_restrict<SLOW>(tl, L, C, bad);
+        tail_restrict<SLOW>(tl, C, L.w, bad);
         L = C;
-        tail_sweep<SLOW, 1>(tl, L.o + L.n0, L.n1, L.w, bad);
+        sweep(true);
     }
-    // the coarsest level's other seven half-sweeps (it has at most 4 cells, unless it is the first)
+    // the coarsest level's other seven half-sweeps
 #pragma unroll 1
-    for (int k = 0; k < 7; k++) {
-        const bool odd = k & 1;
-        if (last > 0) tail_sweep<SLOW, 1>(tl, odd ? L.o + L.n0 : L.o, odd ? L.n1 : L.n0, L.w, bad);
-        else tail_sweep<SLOW, kTailJ>(tl, odd ? L.o + L.n0 : L.o, odd ? L.n1 : L.n0, L.w, bad);
-    }
+    for (int k = 0; k < 7; k++) sweep(k & 1);
 #pragma unroll 1
-    for (int l = last - 1; l >= 1; l--) {
+    for (int l = last - 1; l >= 0; l--) {
         const TailLevel C = L;
         L = tl.lv[l];
-        tail_correct<SLOW, 1>(tl, L, C, bad);
-        tail_sweep<SLOW, 1>(tl, L.o, L.n0, L.w, bad);
-    }
-    if (last > 0) {
-        const TailLevel C = L;
-        L = tl.lv[0];
-        tail_correct<SLOW, kTailJ>(tl, L, C, bad);
-        tail_sweep<SLOW, kTailJ>(tl, L.o, L.n0, L.w, bad);
+        if (L.n1 <= NT) tail_correct<SLOW, 1>(tl, L, C, bad);
+        else tail_correct<SLOW, kTailJ>(tl, L, C, bad);
+        sweep(false);
     }
     return bad;
 }
@@ -1667,7 +1678,7 @@ DEV float2* parity_p(const DevScene& d, int it) { return (it & 1) ? d.cgp2 : d.c
 }  // namespace
 
 size_t pressure_smem(const Levels& lv) {
-    return kTileBytes + tail_bytes(tail_cells(lv));
+    return kTileBytes + tail_bytes(tail_cells(lv), lv.w[lv.tail] * lv.h[lv.tail]);
 }
 
 template <class M>
