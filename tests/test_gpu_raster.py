@@ -111,3 +111,16 @@ def test_set_scene_steps_as_set_solids():
         b.step(1, 1 / 240.0)
     pa, pb = a.download_particles(), b.download_particles()
     assert np.array_equal(pa.view(np.uint8), pb.view(np.uint8))
+
+
+@pytest.mark.parametrize("w,h", [(62, 62), (63, 31), (64, 64), (96, 33), (255, 129), (300, 700)])
+def test_union_depth_across_tiles(w, h):
+    """Solids many 32 x 32 tiles wide, whose depths cross tile borders in every direction, and open
+    cells in many small regions, at grids just below, at and above whole tiles."""
+    sc = S.Scene(w, h)
+    sc.add_box([w * 0.5, h * 0.5], [w * 0.45, h * 0.2], angle=0.1)
+    sc.add_circle([w * 0.55, h * 0.6], min(w, h) * 0.3)
+    for k in range(0, w - 40, 24):
+        ring(sc, k + 8, h - 20, k + 20, h - 8)
+    problems, (_, _, region, _) = compare(sc)
+    assert not problems, problems
