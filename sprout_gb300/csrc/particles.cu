@@ -867,7 +867,7 @@ DEV void sadd(int* sacc, int ps, int lx, int ly, int ch, int v) {
     if (lx >= 0 && ly >= 0 && lx < P2G_T && ly < P2G_T) atomicAdd(&sacc[(ly * P2G_T + lx) * ps + ch], v);
 }
 
-__global__ void __launch_bounds__(256) k_p2g(DevScene d) {
+__global__ void __launch_bounds__(512) k_p2g(DevScene d) {
     extern __shared__ int sacc[];
     __shared__ uint32_t row_beg[P2G_HALO_ROWS], row_pre[P2G_HALO_ROWS + 1];
     const DevParams* P = d.P;
@@ -1044,7 +1044,13 @@ void launch_p2g(const DevScene& d, const LaunchCfg& cfg, cudaStream_t st) {
     (void)cfg;
     dim3 tiles((d.W + P2G_T - 1) / P2G_T, (d.H + P2G_T - 1) / P2G_T);
     size_t smem = (size_t)P2G_T * P2G_T * (d.stride + 1) * sizeof(int);
-    k_p2g<<<tiles, 256, smem, st>>>(d);
+    // Few tiles, and of those only some with liquid, leave most SMs one block: more threads then
+    // hide the latency of its chains of shared atomics (384 x 216, 336 tiles: 22.6 us with 256
+    // threads, 16.6 with 512; 128 x 72: 22.0 and 15.8). With four tiles an SM or more the blocks
+    // hide each other's, and fewer threads wait at the tile's ends (512 x 288, 576 tiles: 28.7 and
+    // 30.7; 1600 x 900: 72 and 86).
+    const bool few = tiles.x * tiles.y <= 3 * 152;
+    k_p2g<<<tiles, few ? 512 : 256, smem, st>>>(d);
 }
 
 }  // namespace sprout
