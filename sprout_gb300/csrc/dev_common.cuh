@@ -440,6 +440,12 @@ DEV void ledger_add(unsigned long long* ledger, int entry, float v) {
     atomicAdd(&ledger[entry], (unsigned long long)x);
 }
 
+// The grid barrier's counter back to zero before a persistent solve (one left by a timeout may have
+// stopped mid-barrier), by the kernel before it in the substep.
+DEV void zero_barrier(const DevScene& d) {
+    if ((blockIdx.x | blockIdx.y | threadIdx.x | threadIdx.y) == 0) d.K->bar_count = 0u;
+}
+
 // Warp max of a non-negative float, then an atomicMax of its bits per warp that exceeds the slot
 // as this SM last saw it (the slot only grows in a kernel, so an old value costs at most a
 // needless atomic; an atomic a warp on the one word took k_project on 1600 x 900 cells 48 us, 13

@@ -719,6 +719,7 @@ __global__ void __launch_bounds__(256) k_visc_explicit(DevScene d) {
 // ---- pressure system ---------------------------------------------------------------------
 
 __global__ void __launch_bounds__(256) k_rhs(DevScene d) {
+    zero_barrier(d);
     CELL_XY;
     const DevParams* P = d.P;
     bool mark = false;
@@ -774,6 +775,7 @@ DEV float p_difference(bool lc, bool ln, float pc, float pn, float j) {
 }
 
 __global__ void __launch_bounds__(256) k_project(DevScene d) {
+    zero_barrier(d);
     CELL_XY;
     float m = 0.0f;
     if (cx >= 1 && cy >= 1 && cx < W && cy < H) {

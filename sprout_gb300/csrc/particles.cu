@@ -25,7 +25,16 @@ namespace sprout {
 
 constexpr uint32_t DEAD_KEY = 0xffffffffu;
 
-__global__ void k_step(DevScene d) {
+// The substep length, by one thread; the others clear what the substep counts up (the cells'
+// particles, with heat their heat sums, the crowd list), which as memory sets were two to three
+// more nodes of the substep's chain.
+__global__ void __launch_bounds__(256) k_step(DevScene d, int thermal) {
+    const int k0 = (blockIdx.x * 256 + threadIdx.x) * 4;
+    for (int k = k0; k < min(k0 + 4, d.ncell + 1); k++) d.count[k] = 0u;
+    if (thermal)
+        for (int k = k0; k < min(k0 + 4, d.ncell); k++) d.hcell[k] = make_int2(0, 0);
+    if (k0 != 0) return;
+    d.crowd[0] = 0u;
     const DevParams* P = d.P;
     StepState* S = d.S;
     float u = maxf(minf(__uint_as_float(S->umax_grid), P->ext[0]), __uint_as_float(S->umax_part));
@@ -677,15 +686,13 @@ __global__ void __launch_bounds__(256) k_advance(DevScene d) {
 
 // ---- the sort ---------------------------------------------------------------------------
 
-constexpr int SCAN_BLOCK = 1024;
+constexpr int SCAN_BLOCK = 1024, SCAN_SPAN = 4 * SCAN_BLOCK;   // threads of a block, counts it scans
 
 // Block-wise exclusive scan of count[0..n) into start, block totals into tmp.
-__global__ void __launch_bounds__(SCAN_BLOCK) k_scan_blocks(const uint32_t* count, uint32_t* start, uint32_t* tmp, int n) {
-    __shared__ uint32_t warp_sums[SCAN_BLOCK / 32];
-    int i = blockIdx.x * SCAN_BLOCK + threadIdx.x;
-    uint32_t v = i < n ? count[i] : 0u;
-    uint32_t x = v;
-    int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+// the exclusive sum of the block's x in thread order; *total: of all of them
+DEV uint32_t scan_exclusive(uint32_t x0, uint32_t* warp_sums, uint32_t* total) {
+    uint32_t x = x0;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
         uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
@@ -703,52 +710,58 @@ __global__ void __launch_bounds__(SCAN_BLOCK) k_scan_blocks(const uint32_t* coun
         warp_sums[lane] = s;
     }
     __syncthreads();
-    uint32_t base = wid > 0 ? warp_sums[wid - 1] : 0u;
-    if (i < n) start[i] = base + x - v;
-    if (threadIdx.x == SCAN_BLOCK - 1) tmp[blockIdx.x] = base + x;
+    *total = warp_sums[SCAN_BLOCK / 32 - 1];
+    return (wid > 0 ? warp_sums[wid - 1] : 0u) + x - x0;
 }
 
-// Exclusive scan of the block totals (one block, any count); the grand total is the
-// number of live particles.
-__global__ void __launch_bounds__(SCAN_BLOCK) k_scan_top(uint32_t* tmp, int nb, StepState* S) {
+// The scan in two kernels: each block's own exclusive sums and its total, then to each block the
+// sum of the totals before it, which it adds up itself (four counts a thread keep those few: 352
+// at 1600 x 900, one a thread at 4 million cells). The totals scanned by a kernel of their
+// own were one more node of the chain, 4 us of a substep.
+__global__ void __launch_bounds__(SCAN_BLOCK) k_scan_blocks(const uint32_t* count, uint32_t* start, uint32_t* tmp, int n) {
     __shared__ uint32_t warp_sums[SCAN_BLOCK / 32];
-    __shared__ uint32_t carry;
-    if (threadIdx.x == 0) carry = 0u;
-    __syncthreads();
-    for (int b0 = 0; b0 < nb; b0 += SCAN_BLOCK) {
-        int i = b0 + threadIdx.x;
-        uint32_t v = i < nb ? tmp[i] : 0u;
-        uint32_t x = v;
-        int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-            if (lane >= o) x += y;
-        }
-        if (lane == 31) warp_sums[wid] = x;
-        __syncthreads();
-        if (wid == 0) {
-            uint32_t s = warp_sums[lane];
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                uint32_t y = __shfl_up_sync(0xffffffffu, s, o);
-                if (lane >= o) s += y;
-            }
-            warp_sums[lane] = s;
-        }
-        __syncthreads();
-        uint32_t base = (wid > 0 ? warp_sums[wid - 1] : 0u) + carry;
-        if (i < nb) tmp[i] = base + x - v;
-        __syncthreads();
-        if (threadIdx.x == SCAN_BLOCK - 1) carry = base + x;
-        __syncthreads();
+    const int i = blockIdx.x * SCAN_SPAN + 4 * threadIdx.x;
+    uint4 v = make_uint4(0u, 0u, 0u, 0u);
+    if (i + 3 < n) v = *reinterpret_cast<const uint4*>(count + i);
+    else {
+        if (i < n) v.x = count[i];
+        if (i + 1 < n) v.y = count[i + 1];
+        if (i + 2 < n) v.z = count[i + 2];
     }
-    if (threadIdx.x == 0) S->n_live = carry;
+    uint32_t total;
+    uint4 s;
+    s.x = scan_exclusive(v.x + v.y + v.z + v.w, warp_sums, &total);
+    s.y = s.x + v.x;
+    s.z = s.y + v.y;
+    s.w = s.z + v.z;
+    if (i + 3 < n) *reinterpret_cast<uint4*>(start + i) = s;
+    else {
+        if (i < n) start[i] = s.x;
+        if (i + 1 < n) start[i + 1] = s.y;
+        if (i + 2 < n) start[i + 2] = s.z;
+    }
+    if (threadIdx.x == 0) tmp[blockIdx.x] = total;
 }
 
-__global__ void k_scan_add(uint32_t* start, const uint32_t* tmp, int n) {
-    int i = blockIdx.x * SCAN_BLOCK + threadIdx.x;
-    if (i < n) start[i] += tmp[blockIdx.x];
+// The grand total is the number of live particles.
+__global__ void __launch_bounds__(SCAN_BLOCK) k_scan_add(uint32_t* start, const uint32_t* tmp, int n, StepState* S) {
+    __shared__ uint32_t warp_sums[SCAN_BLOCK / 32];
+    uint32_t mine = 0u, before;
+    for (uint32_t b = threadIdx.x; b < blockIdx.x; b += SCAN_BLOCK) mine += tmp[b];
+    scan_exclusive(mine, warp_sums, &before);
+    if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) S->n_live = before + tmp[blockIdx.x];
+    const int i = blockIdx.x * SCAN_SPAN + 4 * threadIdx.x;
+    if (i + 3 < n) {
+        uint4* p = reinterpret_cast<uint4*>(start + i);
+        uint4 v = *p;
+        v.x += before;
+        v.y += before;
+        v.z += before;
+        v.w += before;
+        *p = v;
+    } else {
+        for (int k = i; k < min(i + 3, n); k++) start[k] += before;
+    }
 }
 
 __global__ void k_place(DevScene d) {
@@ -1015,9 +1028,7 @@ __global__ void __launch_bounds__(512) k_p2g(DevScene d) {
 // ---- launchers ------------------------------------------------------------------------
 
 void launch_advance(const DevScene& d, const LaunchCfg& cfg, cudaStream_t st) {
-    k_step<<<1, 1, 0, st>>>(d);
-    cudaMemsetAsync(d.count, 0, (size_t)(d.ncell + 1) * sizeof(uint32_t), st);
-    if (cfg.thermal) cudaMemsetAsync(d.hcell, 0, (size_t)d.ncell * sizeof(int2), st);
+    k_step<<<d.ncell / 1024 + 1, 256, 0, st>>>(d, cfg.thermal ? 1 : 0);
     uint32_t nb = (cfg.n_slots + 255) / 256;
     if (nb == 0) nb = 1;
     if (cfg.xtra) k_advance<true><<<nb, 256, 0, st>>>(d);
@@ -1028,12 +1039,10 @@ void launch_sort(const DevScene& d, const LaunchCfg& cfg, cudaStream_t st) {
     uint32_t nb = (cfg.n_slots + 255) / 256;
     if (nb == 0) nb = 1;
     int n = d.ncell + 1;
-    int sb = (n + SCAN_BLOCK - 1) / SCAN_BLOCK;
+    int sb = (n + SCAN_SPAN - 1) / SCAN_SPAN;
     k_scan_blocks<<<sb, SCAN_BLOCK, 0, st>>>(d.count, d.start, d.scan_tmp, n);
-    k_scan_top<<<1, SCAN_BLOCK, 0, st>>>(d.scan_tmp, sb, d.S);
-    k_scan_add<<<sb, SCAN_BLOCK, 0, st>>>(d.start, d.scan_tmp, n);
+    k_scan_add<<<sb, SCAN_BLOCK, 0, st>>>(d.start, d.scan_tmp, n, d.S);
     k_place<<<nb, 256, 0, st>>>(d);
-    cudaMemsetAsync(d.crowd, 0, sizeof(uint32_t), st);
     k_cell_sort<<<(d.ncell + 255) / 256, 256, 0, st>>>(d);
     k_crowd_sort<<<kCrowdBlocks, 256, 0, st>>>(d);
     k_cell_gather<<<nb, 256, 0, st>>>(d);

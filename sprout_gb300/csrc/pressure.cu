@@ -2001,8 +2001,7 @@ void launch_frame_end_many(const DevScene* scenes, int n, cudaStream_t st) {
 }
 
 cudaError_t launch_pressure(const DevScene& d, const LaunchCfg& cfg, cudaStream_t st, int second) {
-    // barrier counter back to zero (a solve left by a timeout may have stopped mid-barrier)
-    cudaMemsetAsync(&d.K->bar_count, 0, sizeof(uint32_t), st);
+    // (the right-hand side's kernel, k_rhs or k_rhs_visc, has zeroed the barrier)
     // cg_scale mode 1: with the viscosity between two solves, the first starts from last
     // substep's P1 alone (viscous_warm, mod.rs:2979-2983)
     int scale_mode = (!second && cfg.visc_mode == 2 && cfg.twice && cfg.viscous_warm) ? 1 : 0;

@@ -124,6 +124,7 @@ DEV void couplings(const DevScene& d, int cx, int cy, int i, float4& a, float4& 
 
 // visc_diag.comp:56-119, with the multigrid's level 0 (viscosity_precond 1).
 __global__ void __launch_bounds__(256) k_visc_diag(DevScene d) {
+    zero_barrier(d);
     __shared__ uint32_t s_was;
     const uint32_t slot = blockIdx.y * gridDim.x + blockIdx.x;
     const int t = threadIdx.y * 16 + threadIdx.x;
@@ -1363,6 +1364,7 @@ namespace {
 
 // rhs_visc.comp
 __global__ void __launch_bounds__(256) k_rhs_visc(DevScene d) {
+    zero_barrier(d);
     const int cx = blockIdx.x * 16 + threadIdx.x, cy = blockIdx.y * 16 + threadIdx.y;
     if (cx >= d.W || cy >= d.H) return;
     const int W = d.W;
@@ -1446,7 +1448,7 @@ void launch_viscosity_setup(const DevScene& d, const LaunchCfg& cfg, cudaStream_
 }
 
 cudaError_t launch_viscosity(const DevScene& d, const LaunchCfg& cfg, cudaStream_t st, int restrain) {
-    cudaMemsetAsync(&d.K->bar_count, 0, sizeof(uint32_t), st);
+    // (k_visc_diag, or k_project between two pressure solves, has zeroed the barrier)
     void* args[] = {(void*)&d, &restrain};
     const void* fn = cfg.visc_sweeps >= 2 ? (const void*)k_visc_solve<2> : (const void*)k_visc_solve<1>;
     return cudaLaunchCooperativeKernel(fn, dim3(cfg.visc_blocks), dim3(NT), args, 0, st);
