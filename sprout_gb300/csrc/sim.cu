@@ -119,9 +119,6 @@ struct SproutSim {
         if (stage_done) cudaEventDestroy(stage_done);
         if (exec) cudaGraphExecDestroy(exec);
         if (graph) cudaGraphDestroy(graph);
-        for (cudaEvent_t e : chunk_ev)
-            if (e) cudaEventDestroy(e);
-        if (chunks) cudaFreeHost(chunks);
         for (void* p : allocs) cudaFree(p);
         if (stream) cudaStreamDestroy(stream);
     }
@@ -742,26 +739,16 @@ struct SproutSim {
 
     // ---- many particles from the host to the device ---------------------------------------
     //
-    // A large array is settled by several host threads, each into two small pinned chunks of its
-    // own that the device copies in turn. One thread settling a copy of the array and copying
-    // that from pageable memory took 25 ms for 2.3 million particles (110 MB), 10 ns a particle
-    // to settle and 1 to copy; 16 threads take 6.4 ms, most of it settling. A thread costs about
-    // 30 us to start and takes 32768 particles (0.35 ms) or more; four are the fewest that win.
-    static constexpr uint32_t kPerWorker = 32768, kChunkParticles = 4096;
-    static constexpr int kCopyWorkers = 16, kFewestWorkers = 4;
-    SproutParticle* chunks = nullptr;   // 2 per worker (6 MB, freed with the sim)
-    cudaEvent_t chunk_ev[2 * kCopyWorkers] = {};
-    // (false: no pinned memory to be had, the plain copy serves)
-    bool ensure_chunks() {
-        if (chunks) return true;
-        cudaError_t e = cudaSuccess;
-        for (cudaEvent_t& v : chunk_ev)
-            if (!v && e == cudaSuccess) e = cudaEventCreateWithFlags(&v, cudaEventDisableTiming);
-        if (e == cudaSuccess) e = cudaMallocHost((void**)&chunks, sizeof(SproutParticle) * kChunkParticles * 2 * kCopyWorkers);
-        if (e == cudaSuccess) return true;
-        chunks = nullptr;
-        cudaGetLastError();
-        return false;
+    // A large array is settled by several host threads, each its own part, which also share the
+    // page faults of the fresh copy: one thread took 25 ms for 2.3 million particles (110 MB), 10 ns
+    // a particle to settle and 1 to copy to the device; 16 take 4.6 ms. A thread costs about 30
+    // us to start and takes 16384 particles (0.16 ms) or more.
+    static constexpr uint32_t kPerWorker = 16384;
+    static constexpr int kSettleWorkers = 16;
+    static int settle_workers(uint32_t n) {
+        cpu_set_t cpus;   // those this process may run on: threads sharing one are slower than one alone
+        const int have = sched_getaffinity(0, sizeof cpus, &cpus) == 0 ? CPU_COUNT(&cpus) : 1;
+        return std::max(1, std::min({have, (int)(n / kPerWorker), (int)kSettleWorkers}));
     }
     // f(w) for every worker w, on threads of their own where there are any to be had
     template <class F>
@@ -777,92 +764,48 @@ struct SproutSim {
         for (; w < workers; w++) f(w);
         for (std::thread& t : ts) t.join();
     }
-    static int copy_workers(uint32_t n) {
-        cpu_set_t cpus;   // those this process may run on: threads sharing one are slower than one alone
-        const int have = sched_getaffinity(0, sizeof cpus, &cpus) == 0 ? CPU_COUNT(&cpus) : 1;
-        return std::min({have, (int)(n / kPerWorker), (int)kCopyWorkers});
-    }
-    // chunk c = w, w + workers, ... of n particles: f(first, count, slot), slot the chunk's buffer number
-    template <class F>
-    static void each_chunk(int w, int workers, uint32_t n, F&& f) {
-        int turn = 0;
-        for (uint64_t first = (uint64_t)w * kChunkParticles; first < n; first += (uint64_t)workers * kChunkParticles, turn++)
-            if (!f((uint32_t)first, (uint32_t)std::min<uint64_t>(kChunkParticles, n - first), 2 * w + (turn & 1))) return;
-    }
-    // The materials of settled particles in[0 .. n) with their reset ids; *bad: the first one with a
-    // non-finite position, or n.
-    void scan_particles(const SproutParticle* in, uint32_t n, bool* present, bool* th, uint32_t* bad) const {
-        const int workers = copy_workers(n);
-        bool seen[kCopyWorkers][kMaxMaterials] = {}, hot[kCopyWorkers] = {};
-        uint32_t first_bad[kCopyWorkers];
-        for (uint32_t& b : first_bad) b = n;
+    // in[0 .. n) with ids from 0, settled, into out; their materials added to present and *th.
+    // Returns the first particle with a non-finite position, or n.
+    uint32_t settle_all(const SproutParticle* in, uint32_t n, SproutParticle* out, bool* present, bool* th) const {
+        const int workers = settle_workers(n);
+        struct Part {
+            uint32_t bad;
+            bool present[kMaxMaterials], th;
+        };
+        std::vector<Part> parts(workers);
         each_worker(workers, [&](int w) {
             const uint32_t lo = (uint32_t)((uint64_t)n * w / workers), hi = (uint32_t)((uint64_t)n * (w + 1) / workers);
-            bool mine[kMaxMaterials] = {}, heated = false;   // (a worker's own cache lines)
-            for (uint32_t k = lo; k < hi; k++) {
-                SproutParticle q = in[k];
-                if (!settle_one(q)) {
-                    first_bad[w] = k;
+            Part mine{n, {}, false};   // (on the worker's own stack until it is done)
+            std::copy(in + lo, in + hi, out + lo);
+            uint32_t k = lo;
+            for (SproutParticle* const ps = out; k < hi; k++) {
+                ps[k].id = k;
+                if (!settle_one(ps[k])) {
+                    mine.bad = k;
                     break;
                 }
-                mark_materials(&q, 1, mine, &heated);
             }
-            std::copy(mine, mine + kMaxMaterials, seen[w]);
-            hot[w] = heated;
+            if (k == hi) mark_materials(out + lo, hi - lo, mine.present, &mine.th);
+            parts[w] = mine;
         });
-        *bad = n;
-        for (int w = 0; w < workers; w++) {
-            *bad = std::min(*bad, first_bad[w]);
-            *th |= hot[w];
-            for (int m = 0; m < kMaxMaterials; m++) present[m] |= seen[w][m];
+        uint32_t bad = n;
+        for (const Part& p : parts) {
+            bad = std::min(bad, p.bad);
+            *th |= p.th;
+            for (int m = 0; m < kMaxMaterials; m++) present[m] |= p.present[m];
         }
+        return bad;
     }
-    // in[0 .. n), settled, with ids from 0, into d.part, by way of the chunks (ensure_chunks).
-    int upload_settled(const SproutParticle* in, uint32_t n) {
-        const int workers = copy_workers(n);
-        cudaError_t err[kCopyWorkers] = {};
-        each_worker(workers, [&](int w) {
-            cudaError_t& e = err[w];
-            if ((e = cudaSetDevice(device)) != cudaSuccess) return;
-            each_chunk(w, workers, n, [&](uint32_t first, uint32_t count, int slot) {
-                SproutParticle* q = chunks + (size_t)slot * kChunkParticles;
-                if ((e = cudaEventSynchronize(chunk_ev[slot])) != cudaSuccess) return false;   // its last copy
-                for (uint32_t k = 0; k < count; k++) {
-                    q[k] = in[first + k];
-                    q[k].id = first + k;
-                    settle_one(q[k]);
-                }
-                e = cudaMemcpyAsync(d.part + 3 * (size_t)first, q, (size_t)count * sizeof(SproutParticle), cudaMemcpyHostToDevice, stream);
-                if (e == cudaSuccess) e = cudaEventRecord(chunk_ev[slot], stream);
-                return e == cudaSuccess;
-            });
-        });
-        const cudaError_t done = cudaStreamSynchronize(stream);
-        for (cudaError_t e : err) CUDA_TRY(e);
-        CUDA_TRY(done);
-        return SPROUT_OK;
-    }
+
     int reset(const SproutParticle* in, uint32_t n) {
         if (n > capacity) n = capacity;
         bool present[kMaxMaterials] = {};
         bool th = solids_heated;
-        std::vector<SproutParticle> ps;   // settled here, unless there are many
-        const bool many = copy_workers(n) >= kFewestWorkers && ensure_chunks();
-        if (many) {
-            uint32_t bad = n;
-            scan_particles(in, n, present, &th, &bad);
-            if (bad < n) {
-                SproutParticle q = in[bad];
-                return settle(q, bad);
-            }
-        } else {
-            ps.assign(in, in + n);
-            for (uint32_t k = 0; k < n; k++) {
-                ps[k].id = k;
-                int rc = settle(ps[k], k);
-                if (rc != SPROUT_OK) return rc;
-            }
-            mark_materials(ps.data(), n, present, &th);
+        const std::unique_ptr<SproutParticle[]> ps(new SproutParticle[std::max(n, 1u)]);
+        const uint32_t bad = settle_all(in, n, ps.get(), present, &th);
+        if (bad < n) {
+            SproutParticle q = in[bad];
+            return settle(q, bad);
         }
         if (std::fabs(params.ambient_temp - kTRef) > 0.05f) th = true;
         int rc = set_tank(present, th);
@@ -880,11 +823,7 @@ struct SproutSim {
         d.stride = std::max(tank.stride, 8);
         CUDA_TRY(cudaStreamSynchronize(stream));
         size_t nc = (size_t)W * H;
-        if (many) {
-            if ((rc = upload_settled(in, n)) != SPROUT_OK) return rc;
-        } else if (n > 0) {
-            CUDA_TRY(cudaMemcpy(d.part, ps.data(), (size_t)n * sizeof(SproutParticle), cudaMemcpyHostToDevice));
-        }
+        if (n > 0) CUDA_TRY(cudaMemcpy(d.part, ps.get(), (size_t)n * sizeof(SproutParticle), cudaMemcpyHostToDevice));
         CUDA_TRY(cudaMemset(d.pres, 0, nc * sizeof(float2)));
         CUDA_TRY(cudaMemset(d.p2keep, 0, nc * sizeof(float)));
         CUDA_TRY(cudaMemset(d.S, 0, sizeof(StepState)));

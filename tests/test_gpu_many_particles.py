@@ -1,6 +1,6 @@
-"""Large particle arrays (settled in chunks by several threads) against the same
-particles in arrays small enough for the plain copy, byte for byte, at counts around the
-chunk's and the threshold's edges; and the error for a non-finite position."""
+"""Large particle arrays (settled by several threads) against the same particles in arrays that
+one thread settles, byte for byte, at counts around the thresholds' edges; and the error for a
+non-finite position."""
 import numpy as np
 import pytest
 
@@ -27,18 +27,18 @@ def engine(n):
     return S.FluidSim(W, H, n, S.SimParams({"cell_size": 0.002, "tension_water": 0.0, "tension_honey": 0.0}))
 
 
-@pytest.mark.parametrize("n", [131071, 131072, 131073, 163840, 200001, 600001])
-def test_reset_in_chunks(n):
+@pytest.mark.parametrize("n", [32767, 32768, 32769, 65537, 163840, 262145, 160001])
+def test_reset_in_parts(n):
     p = some(n)
-    big, small = engine(n), engine(60000)
+    big, small = engine(n), engine(16000)
     big.reset(p)
     got = big.download_particles()
     assert len(got) == n and np.array_equal(got["id"], np.arange(n, dtype=got["id"].dtype))
-    for k in range(0, n, 60000):
-        small.reset(p[k:k + 60000])
+    for k in range(0, n, 16000):
+        small.reset(p[k:k + 16000])
         want = small.download_particles()
         want["id"] += np.uint32(k)
-        assert want.tobytes() == got[k:k + 60000].tobytes(), k
+        assert want.tobytes() == got[k:k + 16000].tobytes(), k
 
 
 def test_the_first_non_finite_position_is_named_and_nothing_changes():
