@@ -209,55 +209,85 @@ DEV void cg_scale_tile(const DevScene& d, int t, int mode) {
     }
 }
 
-// mg_build.comp on tile t of coarse level l + 1, from level l.
+// mg_build.comp's aggregation: a coarse cell's diagonal D and couplings A from its four fine cells
+// and their neighbours. dg(x, y), x and y from -1 to 2: the fine cell's diagonal, 0 where there is
+// no unknown; row(x, y): its couplings. Everything is loaded before any of it is used: a load at a
+// time behind its neighbour's test was 24 latencies in a row.
+template <class Dg, class Row>
+DEV void galerkin(Dg&& dg, Row&& row, float& D, float4& A) {
+    float c[2][2], l[2], r[2], b[2], t[2];
+    float4 w[2][2];
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+        l[k] = dg(-1, k);
+        r[k] = dg(2, k);
+        b[k] = dg(k, -1);
+        t[k] = dg(k, 2);
+#pragma unroll
+        for (int x = 0; x < 2; x++) {
+            c[k][x] = dg(x, k);
+            w[k][x] = row(x, k);
+        }
+    }
+    D = 0.0f;
+    A = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+    for (int y = 0; y < 2; y++)
+#pragma unroll
+        for (int x = 0; x < 2; x++) {
+            if (!(c[y][x] > 0.0f)) continue;
+            const float4 v = w[y][x];
+            D += c[y][x];
+            if (x == 1) { if (c[y][0] > 0.0f) D -= v.x; }
+            else if (l[y] > 0.0f) A.x += v.x;
+            if (x == 0) { if (c[y][1] > 0.0f) D -= v.y; }
+            else if (r[y] > 0.0f) A.y += v.y;
+            if (y == 1) { if (c[0][x] > 0.0f) D -= v.z; }
+            else if (b[x] > 0.0f) A.z += v.z;
+            if (y == 0) { if (c[1][x] > 0.0f) D -= v.w; }
+            else if (t[x] > 0.0f) A.w += v.w;
+        }
+    if (!(D > 1e-7f)) {
+        D = 0.0f;
+        A = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    }
+}
+
+// mg_build.comp on tile t of coarse level l + 1, from level l. One tile is two latencies, its flags'
+// and its cells' (galerkin); the three levels of a 384 x 216 tank took 6, 6 and 5 us, 2.9, 2.3 and 2.1 now.
 template <class M>
 DEV void mg_build_tile(const DevScene& d, int l, int t) {
     const Lv F = lev(d.lv, l), C = lev(d.lv, l + 1);
     const int tfx = tiles_x(F), tfy = tiles_y(F), tcx = tiles_x(C);
-    __shared__ uint32_t s_state;
-    const int tx = t % tcx, ty = t / tcx;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        uint32_t on = 0u;
-        for (int k = 0; k < 4; k++) {
-            int fx = 2 * tx + (k & 1), fy = 2 * ty + (k >> 1);
-            if (fx < tfx && fy < tfy) on |= d.ptile[F.toff + fy * tfx + fx];
-        }
-        uint32_t slot = (uint32_t)C.toff + (uint32_t)t;
-        uint32_t was = d.ptile[slot];
-        d.ptile[slot] = on != 0u ? 1u : 0u;
-        s_state = (on != 0u ? 1u : 0u) | (was != 0u ? 2u : 0u);
+    const int ty = qdiv(t, C.tm), tx = t - ty * tcx;
+    const uint32_t slot = (uint32_t)C.toff + (uint32_t)t, was = d.ptile[slot];
+    uint32_t on = 0u;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const int fx = 2 * tx + (k & 1), fy = 2 * ty + (k >> 1);
+        if (fx < tfx && fy < tfy) on |= d.ptile[F.toff + fy * tfx + fx];
     }
-    __syncthreads();
-    const uint32_t state = s_state;
-    if (state == 0u) return;
+    __syncthreads();   // every thread has read what the first one writes
+    if (threadIdx.x == 0) d.ptile[slot] = on != 0u ? 1u : 0u;
     const int Cx = tx * 16 + (threadIdx.x & 15), Cy = ty * 16 + (threadIdx.x >> 4);
-    if (Cx >= C.w || Cy >= C.h) return;
+    if ((on | was) == 0u || Cx >= C.w || Cy >= C.h) return;
     const int o = l_at(C, Cx, Cy);
-    if ((state & 1u) == 0u) {
-        M::setA(d, o, make_float4(0.0f, 0.0f, 0.0f, 0.0f), 0.0f);
-        return;
-    }
     float D = 0.0f;
     float4 A = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    for (int k = 0; k < 4; k++) {
-        int cx = 2 * Cx + (k & 1), cy = 2 * Cy + (k >> 1);
-        if (!unknown<M>(d, F, cx, cy)) continue;
-        int i = l_at(F, cx, cy);
-        D += M::Dg(d, i);
-        float4 w = M::A(d, i);
-        for (int q = 0; q < 4; q++) {
-            int nx = cx + NBX[q], ny = cy + NBY[q];
-            if (!unknown<M>(d, F, nx, ny)) continue;
-            float wd = wcomp(w, q);
-            if ((nx >> 1) == Cx && (ny >> 1) == Cy) D -= wd;
-            else if (q == 0) A.x += wd;
-            else if (q == 1) A.y += wd;
-            else if (q == 2) A.z += wd;
-            else A.w += wd;
-        }
-    }
-    M::setA(d, o, D > 1e-7f ? A : make_float4(0.0f, 0.0f, 0.0f, 0.0f), D > 1e-7f ? D : 0.0f);
+    if (on != 0u)
+        galerkin(
+            [&](int x, int y) {
+                x += 2 * Cx;
+                y += 2 * Cy;
+                return l_inside(F, x, y) ? M::Dg(d, l_at(F, x, y)) : 0.0f;
+            },
+            [&](int x, int y) {
+                x += 2 * Cx;
+                y += 2 * Cy;
+                return l_inside(F, x, y) ? M::A(d, l_at(F, x, y)) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            },
+            D, A);
+    M::setA(d, o, A, D);
 }
 
 // cg_init.comp on level-0 tile t: r = b - A x (the FP32 operator), the tile's sum of b.b
@@ -338,8 +368,6 @@ struct Tail {
     int base, T, nf, nl;
 };
 
-DEV bool t_unknown(const Tail& tl, const Lv& L, int x, int y) { return l_inside(L, x, y) && tl.dy[L.off - tl.base + y * L.w + x].x > 0.0f; }
-
 // A tail of T cells, the first nf of them its first level's, in nl levels, laid out in shared
 // memory at smem; its right-hand sides, live only inside the tail phase, at r.
 DEV Tail tail_at(unsigned char* smem, float2* r, int base, int T, int nf, int nl) {
@@ -384,6 +412,95 @@ __host__ __device__ inline size_t tail_bytes(int T, int nf) {
             (size_t)(T - nf) * 4 * sizeof(uint16_t) + 15) / 16 * 16;
 }
 
+// The lists of the tail's unknowns by colour, of its first level or of all the others at once (a
+// pass has the latency of a chain of shared accesses, a level at a time that was paid per level).
+// An entry's place among its colour does not matter to a half-sweep: the first level's warps
+// count their cells and add once for each colour (an add a cell waited for its turn). The
+// couplings and diagonals so far lie by slot, so they move through registers.
+template <bool FIRST>
+DEV void tail_lists(const Tail& tl, uint16_t* ent) {
+    constexpr int PER = 6;   // the first level has at most 1500 cells, the others together fewer than that
+    const int s0 = FIRST ? 0 : tl.nf, s1 = FIRST ? tl.nf : tl.T;
+    // a cell's place among its colour, from the list's end if odd, under its level and the mask of
+    // its neighbours that are unknowns; none: no unknown
+    constexpr uint32_t kNone = 0xffffffffu, kOdd = 0x8000u;
+    uint32_t p[PER];
+#pragma unroll
+    for (int j = 0; j < PER; j++) {
+        const int s = s0 + (int)threadIdx.x + j * NT;
+        p[j] = kNone;
+        int l = 0;
+        bool odd = false;
+        if (s < s1) {
+            if (!FIRST) {
+                l = 1;
+                while (l + 1 < tl.nl && s >= tl.lv[l + 1].o) l++;
+            }
+            const TailLevel& Q = tl.lv[l];
+            const int t = s - Q.o, y = qdiv(t, Q.wm), x = t - y * Q.w;
+            odd = (x + y) & 1;
+            const uint32_t m = (x > 0 && tl.dy[s - 1].x > 0.0f ? 1u : 0u) | (x + 1 < Q.w && tl.dy[s + 1].x > 0.0f ? 2u : 0u) |
+                               (y > 0 && tl.dy[s - Q.w].x > 0.0f ? 4u : 0u) | (y + 1 < Q.h && tl.dy[s + Q.w].x > 0.0f ? 8u : 0u);
+            if (tl.dy[s].x > 0.0f) p[j] = (uint32_t)l << 20 | m << 16;
+            tl.x[s] = make_float2(0.0f, 0.0f);
+        }
+        const bool on = p[j] != kNone;
+        TailLevel& Q = tl.lv[l];
+        if (FIRST) {
+            const uint32_t even_m = __ballot_sync(0xffffffffu, on && !odd), odd_m = __ballot_sync(0xffffffffu, on && odd);
+            const int lane = threadIdx.x & 31;
+            int e = 0, o = 0;
+            if (lane == 0) {
+                if (even_m) e = atomicAdd(&Q.n0, __popc(even_m));
+                if (odd_m) o = atomicAdd(&Q.n1, __popc(odd_m));
+            }
+            e = __shfl_sync(0xffffffffu, e, 0);
+            o = __shfl_sync(0xffffffffu, o, 0);
+            const uint32_t before = (1u << lane) - 1u;
+            if (on) p[j] |= odd ? kOdd | (uint32_t)(o + __popc(odd_m & before)) : (uint32_t)(e + __popc(even_m & before));
+        } else if (on) {
+            p[j] |= odd ? kOdd | (uint32_t)atomicAdd(&Q.n1, 1) : (uint32_t)atomicAdd(&Q.n0, 1);
+        }
+    }
+    float4 a[PER];
+#pragma unroll
+    for (int j = 0; j < PER; j++) {
+        if (p[j] == kNone) continue;
+        a[j] = tl.a[s0 + (int)threadIdx.x + j * NT];
+        if (!(p[j] & 1u << 16)) a[j].x = 0.0f;
+        if (!(p[j] & 2u << 16)) a[j].y = 0.0f;
+        if (!(p[j] & 4u << 16)) a[j].z = 0.0f;
+        if (!(p[j] & 8u << 16)) a[j].w = 0.0f;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < PER; j++) {   // the entry: the odd cells follow the even ones
+        const int s = s0 + (int)threadIdx.x + j * NT;
+        if (p[j] == kNone) {
+            if (s < s1) ent[s] = (uint16_t)kNoEntry;
+            continue;
+        }
+        const TailLevel& Q = tl.lv[p[j] >> 20];
+        const uint32_t k = p[j] & (kOdd - 1u);
+        const uint32_t e = (uint32_t)Q.o + ((p[j] & kOdd) ? (uint32_t)(Q.n0 + Q.n1) - 1u - k : k);
+        p[j] = e;
+        tl.a[e] = a[j];
+        tl.slot[e] = (uint16_t)s;
+        ent[s] = (uint16_t)e;
+    }
+    float2 dy[PER];
+#pragma unroll
+    for (int j = 0; j < PER; j++) {
+        if (p[j] == kNone) continue;
+        const float D = tl.dy[s0 + (int)threadIdx.x + j * NT].x;
+        dy[j] = make_float2(D, recip(D));
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < PER; j++)
+        if (p[j] != kNone) tl.dy[p[j]] = dy[j];
+}
+
 // mg_tail.comp mode 1 in every block's shared memory, once per solve: the first tail
 // level's matrix from global memory, then the Galerkin matrices of the coarser tail levels
 // (the arithmetic of mg_build.comp). Block 0 also stores them for inspection.
@@ -403,70 +520,30 @@ DEV void tail_setup(const DevScene& d, const Tail& tl, bool writer) {
         const int o = F.off - tl.base, oc = C.off - tl.base;
         for (int t = threadIdx.x; t < C.w * C.h; t += NT) {
             const int ccy = qdiv(t, C.wm), ccx = t - ccy * C.w;
-            float D = 0.0f;
-            float4 A = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            for (int k = 0; k < 4; k++) {
-                int cx = 2 * ccx + (k & 1), cy = 2 * ccy + (k >> 1);
-                if (!t_unknown(tl, F, cx, cy)) continue;
-                int i = o + cy * F.w + cx;
-                D += tl.dy[i].x;
-                float4 w = tl.a[i];
-                for (int q = 0; q < 4; q++) {
-                    int nx = cx + NBX[q], ny = cy + NBY[q];
-                    if (!t_unknown(tl, F, nx, ny)) continue;
-                    float wd = wcomp(w, q);
-                    if ((nx >> 1) == ccx && (ny >> 1) == ccy) D -= wd;
-                    else if (q == 0) A.x += wd;
-                    else if (q == 1) A.y += wd;
-                    else if (q == 2) A.z += wd;
-                    else A.w += wd;
-                }
-            }
-            tl.dy[oc + t].x = D > 1e-7f ? D : 0.0f;
-            tl.a[oc + t] = D > 1e-7f ? A : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            if (writer) M::setA(d, C.off + t, tl.a[oc + t], tl.dy[oc + t].x);
+            float D;
+            float4 A;
+            galerkin(
+                [&](int x, int y) {
+                    x += 2 * ccx;
+                    y += 2 * ccy;
+                    return l_inside(F, x, y) ? tl.dy[o + y * F.w + x].x : 0.0f;
+                },
+                [&](int x, int y) {
+                    x += 2 * ccx;
+                    y += 2 * ccy;
+                    return l_inside(F, x, y) ? tl.a[o + y * F.w + x] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                },
+                D, A);
+            tl.dy[oc + t].x = D;
+            tl.a[oc + t] = A;
+            if (writer) M::setA(d, C.off + t, A, D);
         }
         __syncthreads();
     }
-    // the lists (an entry's place among its colour does not matter to a half-sweep): the couplings
-    // and diagonals so far lie by slot, so they move through registers, level by level; ent: a
-    // slot's entry, kept where the right-hand sides will be
+    // the lists; ent: a slot's entry, kept where the right-hand sides will be
     uint16_t* const ent = reinterpret_cast<uint16_t*>(tl.r);
-    for (int l = 0; l < tl.nl; l++) {
-        const Lv L = lev(d.lv, d.lv.tail + l);
-        TailLevel& Q = tl.lv[l];
-        constexpr int PER = 6;   // a first tail level has at most 1500 cells
-        float4 a[PER];
-        float2 dy[PER];
-        int p[PER];
-        for (int j = 0; j < PER; j++) {
-            const int t = threadIdx.x + j * NT;
-            if (t >= Q.n) break;
-            const int y = qdiv(t, L.wm), x = t - y * L.w, s = Q.o + t;
-            a[j] = tl.a[s];
-            dy[j] = make_float2(tl.dy[s].x, recip(tl.dy[s].x));
-            if (!t_unknown(tl, L, x - 1, y)) a[j].x = 0.0f;
-            if (!t_unknown(tl, L, x + 1, y)) a[j].y = 0.0f;
-            if (!t_unknown(tl, L, x, y - 1)) a[j].z = 0.0f;
-            if (!t_unknown(tl, L, x, y + 1)) a[j].w = 0.0f;
-            p[j] = -1;
-            if (dy[j].x > 0.0f) p[j] = ((x + y) & 1) ? Q.n - 1 - atomicAdd(&Q.n1, 1) : atomicAdd(&Q.n0, 1);
-            tl.x[s] = make_float2(0.0f, 0.0f);
-        }
-        __syncthreads();
-        const int gap = Q.n - Q.n1 - Q.n0;   // the odd cells, so far at the list's end, follow the even ones
-        for (int j = 0; j < PER; j++) {
-            const int t = threadIdx.x + j * NT;
-            if (t >= Q.n) break;
-            int e = p[j];
-            if (e >= Q.n0) e -= gap;
-            ent[Q.o + t] = e < 0 ? (uint16_t)kNoEntry : (uint16_t)(Q.o + e);
-            if (e < 0) continue;
-            tl.a[Q.o + e] = a[j];
-            tl.dy[Q.o + e] = dy[j];
-            tl.slot[Q.o + e] = (uint16_t)(Q.o + t);
-        }
-    }
+    tail_lists<true>(tl, ent);
+    tail_lists<false>(tl, ent);
     __syncthreads();
     for (int l = 1; l < tl.nl; l++) {
         const TailLevel F = tl.lv[l - 1], C = tl.lv[l];
@@ -478,6 +555,10 @@ DEV void tail_setup(const DevScene& d, const Tail& tl, bool writer) {
     }
     __syncthreads();
 }
+// ... of a batch's scene, called: inlined at both of the batch's places it took the registers of the
+// passes around them
+template <class M>
+__device__ __noinline__ void tail_setup_of(const DevScene* d) { tail_setup<M>(*d, make_tail(*d), false); }
 
 // ---- the level passes ---------------------------------------------------------------------------
 //
@@ -1743,7 +1824,7 @@ __global__ void __launch_bounds__(NT, 2) k_mgpcg_batch(BatchView B, int second) 
     // one tail per block stays in its shared memory for the whole solve; with more scenes than
     // blocks, each tail phase sets its tail up again
     const bool resident = B.ns <= (int)gridDim.x;
-    if (resident && (int)blockIdx.x < B.ns) tail_setup<M>(B.scenes[blockIdx.x], make_tail(B.scenes[blockIdx.x]), false);
+    if (resident && (int)blockIdx.x < B.ns) tail_setup_of<M>(B.scenes + blockIdx.x);
     const Geo geom = geo();
     auto of = [&B](int s) -> const DevScene& { return B.scenes[s]; };
     auto item = [&](int l, int k) { return my_item(tc, l, k, [&](uint32_t g) { return batch_item(B, l, (int)g); }); };
@@ -1779,7 +1860,7 @@ __global__ void __launch_bounds__(NT, 2) k_mgpcg_batch(BatchView B, int second) 
             if (fused && !running(s, it)) continue;
             const DevScene& d = B.scenes[s];
             const Tail tl = make_tail(d);
-            if (!resident) tail_setup<M>(d, tl, false);
+            if (!resident) tail_setup_of<M>(&d);
             phase_tail(d.mgr + tl.base, d.mgz + tl.base, tl);
             __syncthreads();
         }
