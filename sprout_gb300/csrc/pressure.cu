@@ -191,6 +191,8 @@ DEV void cg_scale_tile(const DevScene& d, int t, int mode) {
     const int cx = (t % tiles_x(F)) * 16 + (threadIdx.x & 15), cy = (t / tiles_x(F)) * 16 + (threadIdx.x >> 4);
     if (!l_inside(F, cx, cy)) return;
     const int i = l_at(F, cx, cy);
+    const uint32_t active = d.ptile[F.toff + t];
+    const float2 pres = d.pres[i];   // (with the rest, before any is used)
     if (M::kMixed) {
         int m = 0;
         for (int q = 0; q < 4; q++) m |= unknown_op(d, F, cx + NBX[q], cy + NBY[q]) ? (1 << q) : 0;
@@ -198,9 +200,9 @@ DEV void cg_scale_tile(const DevScene& d, int t, int mode) {
     } else {
         d.mgy[i] = make_float2(d.mgd[i], recip_row(d.mgd[i], d.mga[i]));
     }
-    if (d.ptile[F.toff + t] == 0u) return;
+    if (active == 0u) return;
     if (d.mgd[i] > 0.0f) {
-        float p = d.pres[i].x;
+        float p = pres.x;
         if (mode == 1) p -= d.p2keep[i];
         else d.p2keep[i] = 0.0f;
         d.pres[i].x = p * ratio;
@@ -290,48 +292,69 @@ DEV void mg_build_tile(const DevScene& d, int l, int t) {
     M::setA(d, o, A, D);
 }
 
-// cg_init.comp on level-0 tile t: r = b - A x (the FP32 operator), the tile's sum of b.b
-// into part[n + t] (or, with `rr`, of r.r into part[t]).
-template <class M>
-DEV void residual_tile(const DevScene& d, int t, float2* r0, typename M::acc4* buf, bool rr) {
-    using acc = typename M::acc;
-    const Lv F = lev(d.lv, 0);
-    const int n = d.nwg;
-    typename M::acc4* part = M::part(d) + (rr ? 0 : n);
-    if (d.ptile[F.toff + t] == 0u) {
-        if (threadIdx.x == 0) part[t] = M::zero4();
-        return;
-    }
-    const int cx = (t % tiles_x(F)) * 16 + (threadIdx.x & 15), cy = (t / tiles_x(F)) * 16 + (threadIdx.x >> 4);
-    typename M::acc4 a4 = M::zero4();
-    if (l_inside(F, cx, cy)) {
-        const int i = l_at(F, cx, cy);
-        const float D = d.mgd[i];
-        if (D > 0.0f) {
-            float2 x = d.pres[i];
-            float4 w = d.mga[i];
-            float axx = D * x.x, axy = D * x.y;
+// The tree of reduce.glsl:5-14 over a tile's 256 float4 by one warp (tile_tree's order).
+DEV float4 tile_tree4(const float4* v) {
+    const int x = threadIdx.x & 15, h = (threadIdx.x >> 4) & 1;
+    auto b = [&](int j) { return add4(add4(v[j * 16 + x], v[(j + 8) * 16 + x]), add4(v[(j + 4) * 16 + x], v[(j + 12) * 16 + x])); };
+    float4 s = add4(b(h), b(h + 2));
+#pragma unroll
+    for (int k = 16; k > 0; k >>= 1) s = add4(s, shfl_down4(s, k));
+    return s;
+}
+// cg_init.comp over this block's `count` active level-0 tiles (at(k, t): the k-th's scene, its tile
+// in t): r = b - A x (the FP32 operator) and the tile's sum of b.b in the partials' second half. A
+// cell's loads are all issued before the first is used, and one warp adds up a tile's products
+// while the others go on to the next, in the other of two buffers at sums. A load at a time behind
+// its neighbour's test, and a tree of the whole block, the phase (beside it a few blocks set up
+// their tails) took 29 us at 1600 x 900, 20 now.
+template <class M, class At>
+DEV void residual_pass(int count, float4* sums, At&& at) {
+    static_assert(std::is_same<typename M::acc4, float4>::value, "the products are float4");
+    for (int k = 0; k < count; k++) {
+        int t;
+        const DevScene& d = at(k, t);
+        const Lv F = lev(d.lv, 0);
+        const int2 og = tile_origin(F, t);
+        const int cx = og.x + (threadIdx.x & 15), cy = og.y + (threadIdx.x >> 4);
+        float4 a4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (l_inside(F, cx, cy)) {
+            const int i = l_at(F, cx, cy);
+            const float D = d.mgd[i];
+            const float4 w = d.mga[i], b = d.prhs[i];
+            const float2 x = d.pres[i];
+            float nd[4];
+            float2 np[4];
+#pragma unroll
             for (int q = 0; q < 4; q++) {
-                int nx = cx + NBX[q], ny = cy + NBY[q];
-                if (unknown_op(d, F, nx, ny)) {
-                    float wd = wcomp(w, q);
-                    float2 pn = d.pres[l_at(F, nx, ny)];
-                    axx -= wd * pn.x;
-                    axy -= wd * pn.y;
-                }
+                const int nx = cx + NBX[q], ny = cy + NBY[q];
+                const bool in = l_inside(F, nx, ny);
+                const int j = in ? l_at(F, nx, ny) : i;
+                nd[q] = in ? d.mgd[j] : 0.0f;
+                np[q] = d.pres[j];
             }
-            float4 b = d.prhs[i];
-            const float2 r = make_float2(b.x - axx, b.y - axy);
-            r0[i] = r;
-            if (rr) a4 = M::prod4(0.0f, 0.0f, 0.0f, 0.0f, r.x, r.x, r.y, r.y);
-            else a4 = M::prod4(b.x, b.x, b.y, b.y, 0.0f, 0.0f, 0.0f, 0.0f);
-        } else {
-            r0[i] = make_float2(0.0f, 0.0f);
+            float2 r = make_float2(0.0f, 0.0f);
+            if (D > 0.0f) {
+                float axx = D * x.x, axy = D * x.y;
+#pragma unroll
+                for (int q = 0; q < 4; q++)
+                    if (nd[q] > 0.0f) {
+                        const float wd = wcomp(w, q);
+                        axx -= wd * np[q].x;
+                        axy -= wd * np[q].y;
+                    }
+                r = make_float2(b.x - axx, b.y - axy);
+                a4 = M::prod4(b.x, b.x, b.y, b.y, 0.0f, 0.0f, 0.0f, 0.0f);
+            }
+            d.mgr[i] = r;
+        }
+        float4* const buf = sums + (k & 1) * NT;
+        buf[threadIdx.x] = a4;
+        __syncthreads();
+        if (threadIdx.x >= 7 * 32) {
+            const float4 v = tile_tree4(buf);
+            if (threadIdx.x == 7 * 32) M::part(d)[d.nwg + t] = v;
         }
     }
-    buf[threadIdx.x] = a4;
-    block_tree(buf);
-    if (threadIdx.x == 0) part[t] = buf[0];
     __syncthreads();
 }
 
@@ -1249,18 +1272,16 @@ DEV void phase_tail(const float2* R, float2* Z, const Tail& tl) {
 }
 
 // The active-tile lists of levels 0 .. tail - 1 of scene d (one block), from ptile.
-DEV void build_plists(const DevScene& d) {
-    for (int l = 0; l < d.lv.tail; l++) {
-        const Lv L = lev(d.lv, l);
-        compact_flags(d.ptile + L.toff, tiles_x(L) * tiles_y(L), d.plist + L.toff, d.pcount + l);
-    }
+DEV void build_plist(const DevScene& d, int l) {
+    const Lv L = lev(d.lv, l);
+    compact_flags(d.ptile + L.toff, tiles_x(L) * tiles_y(L), d.plist + L.toff, d.pcount + l);
 }
 
 // Level-0 tiles without unknowns keep zero partial sums through the solve (their tile
 // bodies are never run): set them once at its start, every half and precision.
 template <class M>
 DEV void zero_inactive_tile(const DevScene& d, int t) {
-    if (threadIdx.x != 0 || d.ptile[t] != 0u) return;
+    if (d.ptile[t] != 0u) return;
     const int n = d.nwg;
     M::part(d)[t] = M::zero4();
     M::part(d)[n + t] = M::zero4();
@@ -1614,14 +1635,17 @@ __global__ void __launch_bounds__(NT, 2) k_mgpcg(const __grid_constant__ DevScen
         if (!grid_sync(d.K)) return;
     }
     // the active-tile lists (ptile is final now) and the inactive tiles' zero partial sums
-    if (blockIdx.x == 0) build_plists(d);
-    for (int t = blockIdx.x; t < n; t += gridDim.x) zero_inactive_tile<M>(d, t);
+    for (int l = blockIdx.x; l < d.lv.tail; l += gridDim.x) build_plist(d, l);   // a level a block
+    for (int t = blockIdx.x * NT + threadIdx.x; t < n; t += gridDim.x * NT) zero_inactive_tile<M>(d, t);
     if (!grid_sync(d.K)) return;
     fill_cache(d, tc);
     if (tail_reader(d, tc)) tail_setup<M>(d, tl, blockIdx.x == 0);
     float2* r_cur = d.mgr;    // level 0 of mgr: the residual, double-buffered with mgr2
     float2* r_nxt = d.mgr2;
-    for_active(d, 0, tc, [&](int t) { residual_tile<M>(d, t, r_cur, buf, false); });
+    residual_pass<M>(my_count(active_tiles(d, 0, tc)), reinterpret_cast<float4*>(dyn_smem), [&](int k, int& t) -> const DevScene& {
+        t = my_tile(d, tc, 0, k);
+        return d;
+    });
     if (!grid_sync(d.K)) return;
     // b.b now, while nothing writes the second half of the partials: the first apply phase
     // after the V-cycle does, and a block can reach it before a slower one has summed them
@@ -1789,9 +1813,19 @@ __global__ void __launch_bounds__(NT, 2) k_mgpcg_batch(BatchView B, int second) 
         }
         if (!grid_sync(BK)) return;
     }
-    // every scene's active-tile lists (one block each) and the inactive tiles' zero partials
-    for (int s = blockIdx.x; s < B.ns; s += gridDim.x) build_plists(B.scenes[s]);
-    for_tiles(B, 0, [&](int s, const DevScene& d, int t) { zero_inactive_tile<M>(d, t); });
+    // every scene's active-tile lists (a block each level) and the inactive tiles' zero partials
+    for (int g = blockIdx.x; g < B.ns * B.max_tail; g += gridDim.x) {
+        const DevScene& d = B.scenes[g / B.max_tail];
+        const int l = g % B.max_tail;
+        if (l < d.lv.tail) build_plist(d, l);
+    }
+    {
+        const int* o = B.off;
+        for (int g = blockIdx.x * NT + threadIdx.x; g < o[B.ns]; g += gridDim.x * NT) {
+            const int s = scene_of(o, B.ns, g);
+            zero_inactive_tile<M>(B.scenes[s], g - o[s]);
+        }
+    }
     if (!grid_sync(BK)) return;
     // ... and their prefix sums per level over the scenes
     if (blockIdx.x == 0) {
@@ -1808,7 +1842,11 @@ __global__ void __launch_bounds__(NT, 2) k_mgpcg_batch(BatchView B, int second) 
     }
     if (!grid_sync(BK)) return;
     fill_cache_b(B, tc);
-    for_active_b(B, 0, tc, [&](int s, const DevScene& d, int t) { residual_tile<M>(d, t, d.mgr, buf, false); });
+    residual_pass<M>(my_count(active_tiles_b(B, 0, tc)), reinterpret_cast<float4*>(dyn_smem), [&](int k, int& t) -> const DevScene& {
+        const uint32_t g = my_item(tc, 0, k, [&](uint32_t q) { return batch_item(B, 0, (int)q); });
+        t = (int)(g & 0xffffu);
+        return B.scenes[g >> 16];
+    });
     if (!grid_sync(BK)) return;
     // b.b of each scene (before the first apply phase reuses those partials)
     for (int s = blockIdx.x; s < B.ns; s += gridDim.x) {

@@ -320,32 +320,38 @@ static __device__ __noinline__ T total(const T* part, int n, T* buf) {
 }
 
 // One block compacts the nonzero flags[0 .. T) into out (their indices, in order) and
-// stores how many into *count.
+// stores how many into *count. Four flags a thread: a round of a whole block is one load's
+// latency and two barriers (at 1600 x 900 the level-0 flags are 5700).
 DEV void compact_flags(const uint32_t* flags, int T, uint32_t* out, uint32_t* count) {
     __shared__ uint32_t wsum[NT / 32];
-    __shared__ uint32_t s_base;
-    if (threadIdx.x == 0) s_base = 0u;
-    __syncthreads();
-    for (int b0 = 0; b0 < T; b0 += NT) {
-        const int k = b0 + threadIdx.x;
-        const bool on = k < T && flags[k] != 0u;
-        const uint32_t bal = __ballot_sync(0xffffffffu, on);
-        const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-        if (lane == 0) wsum[w] = __popc(bal);
-        __syncthreads();
-        uint32_t before = s_base;
-        for (int j = 0; j < w; j++) before += wsum[j];
-        before += __popc(bal & ((1u << lane) - 1u));
-        if (on) out[before] = (uint32_t)k;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            uint32_t tot = 0;
-            for (int j = 0; j < NT / 32; j++) tot += wsum[j];
-            s_base += tot;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    uint32_t base = 0u;
+    for (int b0 = 0; b0 < T; b0 += 4 * NT) {
+        const int k = b0 + 4 * (int)threadIdx.x;
+        bool on[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) on[q] = k + q < T && flags[k + q] != 0u;
+        const uint32_t mine = (on[0] ? 1u : 0u) + (on[1] ? 1u : 0u) + (on[2] ? 1u : 0u) + (on[3] ? 1u : 0u);
+        uint32_t x = mine;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
         }
+        __syncthreads();   // the last round's sums are read
+        if (lane == 31) wsum[w] = x;
         __syncthreads();
+        uint32_t at = base + x - mine;
+#pragma unroll
+        for (int j = 0; j < NT / 32; j++) {
+            at += j < w ? wsum[j] : 0u;
+            base += wsum[j];
+        }
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+            if (on[q]) out[at++] = (uint32_t)(k + q);
     }
-    if (threadIdx.x == 0) *count = s_base;
+    if (threadIdx.x == 0) *count = base;
     __syncthreads();
 }
 
