@@ -480,39 +480,10 @@ struct VSolve {
         __syncthreads();
     }
 
-    // the compact lists of active tiles per level (block 0)
-    DEV void build_lists(int nlev) const {
-        __shared__ uint32_t wsum[NT / 32];
-        __shared__ uint32_t s_base;
-        for (int l = 0; l <= nlev; l++) {
-            const Lv L = lev(d.lv, l);
-            const int T = tiles_x(L) * tiles_y(L);
-            const uint32_t* flags = l == 0 ? d.tiles : d.vtile + L.toff;
-            uint32_t* out = d.vlist + L.toff;
-            if (threadIdx.x == 0) s_base = 0u;
-            __syncthreads();
-            for (int b0 = 0; b0 < T; b0 += NT) {
-                const int k = b0 + threadIdx.x;
-                const bool on = k < T && flags[k] != 0u;
-                const uint32_t bal = __ballot_sync(0xffffffffu, on);
-                const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-                if (lane == 0) wsum[w] = __popc(bal);
-                __syncthreads();
-                uint32_t before = s_base;
-                for (int j = 0; j < w; j++) before += wsum[j];
-                before += __popc(bal & ((1u << lane) - 1u));
-                if (on) out[before] = (uint32_t)k;
-                __syncthreads();
-                if (threadIdx.x == 0) {
-                    uint32_t tot = 0;
-                    for (int j = 0; j < NT / 32; j++) tot += wsum[j];
-                    s_base += tot;
-                }
-                __syncthreads();
-            }
-            if (threadIdx.x == 0) d.vcount[l] = s_base;
-            __syncthreads();
-        }
+    // the compact list of active tiles of level l (one block)
+    DEV void build_list(int l) const {
+        const Lv L = lev(d.lv, l);
+        compact_flags(l == 0 ? d.tiles : d.vtile + L.toff, tiles_x(L) * tiles_y(L), d.vlist + L.toff, d.vcount + l);
     }
 
     // visc_strain.comp on level-0 tile tt (if active): the weighted strain of the current
@@ -525,20 +496,24 @@ struct VSolve {
         const int cx = og.x + (threadIdx.x & 15), cy = og.y + (threadIdx.x >> 4);
         if (!in_grid(d, cx, cy)) return;
         const int i = cy * W + cx;
-        const float4 w4 = d.vw[i];
+        // (the loads before anything is tested)
+        const int N = W * d.H;
+        const float4 w4 = d.vw[i], me = d.vel[i];
+        const float4 lf = d.vel[max(i - 1, 0)], rt = d.vel[min(i + 1, N - 1)];
+        const float4 dn = d.vel[max(i - W, 0)], up = d.vel[min(i + W, N - 1)];
         float4 o = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        auto vu = [&](int j) { float4 v = d.vel[j]; return face_live(v.z) ? v.x : 0.0f; };
-        auto vv = [&](int j) { float4 v = d.vel[j]; return face_live(v.w) ? v.y : 0.0f; };
+        auto vu = [](const float4& v) { return face_live(v.z) ? v.x : 0.0f; };
+        auto vv = [](const float4& v) { return face_live(v.w) ? v.y : 0.0f; };
         if (w4.x > 0.0f) {
-            o.x = w4.x * (vu(i + 1) - vu(i));
-            o.y = w4.x * (vv(i + W) - vv(i));
+            o.x = w4.x * (vu(rt) - vu(me));
+            o.y = w4.x * (vv(up) - vv(me));
         }
         if (w4.y > 0.0f) {
-            float ua = vu(i), ub = vu(i - W), va = vv(i), vb = vv(i - 1);
-            if (v_closed_u(d, i) && v_live_u(d, i - W)) ua = -ub;
-            if (v_closed_u(d, i - W) && v_live_u(d, i)) ub = -ua;
-            if (v_closed_v(d, i) && v_live_v(d, i - 1)) va = -vb;
-            if (v_closed_v(d, i - 1) && v_live_v(d, i)) vb = -va;
+            float ua = vu(me), ub = vu(dn), va = vv(me), vb = vv(lf);
+            if (face_closed(me.z) && face_live(dn.z)) ua = -ub;
+            if (face_closed(dn.z) && face_live(me.z)) ub = -ua;
+            if (face_closed(me.w) && face_live(lf.w)) va = -vb;
+            if (face_closed(lf.w) && face_live(me.w)) vb = -va;
             o.z = w4.y * 0.5f * ((ua - ub) + (va - vb));
         }
         d.vs[i] = o;
@@ -938,7 +913,7 @@ __global__ void __launch_bounds__(NT, 2) k_visc_solve(DevScene d, int restrain) 
     const int nlev = P->visc_levels;
     VSolve<NU> V{d, sm, K, d.nwg, tc};
     const float tz = P->tol[2];
-    if (blockIdx.x == 0) V.build_lists(nlev);
+    for (int l = blockIdx.x; l <= nlev; l += gridDim.x) V.build_list(l);   // a level a block
     if (restrain) V.strain();
     if (!grid_sync(d.K)) return;
     V.fill_cache(nlev);
@@ -1201,8 +1176,11 @@ __global__ void __launch_bounds__(NT, 2) k_visc_batch(VBatchView B) {
                 if (run(s)) V(s).mgz_finish(tt, g, (par & 1) ? B.scenes[s].vq2 : B.scenes[s].vq, S[s].half); });
     };
 
-    // the lists (one block per tank) and the strain of u* (every tank takes it again)
-    for (int s = blockIdx.x; s < ns; s += gridDim.x) V(s).build_lists(nlev(s));
+    // the lists (a block each level) and the strain of u* (every tank takes it again)
+    for (int g = blockIdx.x; g < ns * (B.max_lev + 1); g += gridDim.x) {
+        const int s = g / (B.max_lev + 1), l = g % (B.max_lev + 1);
+        if (l <= nlev(s)) V(s).build_list(l);
+    }
     for_all0([&](int s, int tt) { V(s).strain_tile(tt); });
     if (!grid_sync(BK)) return;
     // the prefix sums of the active tiles per level over the tanks, and the start
