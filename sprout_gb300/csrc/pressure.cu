@@ -292,15 +292,6 @@ DEV void mg_build_tile(const DevScene& d, int l, int t) {
     M::setA(d, o, A, D);
 }
 
-// The tree of reduce.glsl:5-14 over a tile's 256 float4 by one warp (tile_tree's order).
-DEV float4 tile_tree4(const float4* v) {
-    const int x = threadIdx.x & 15, h = (threadIdx.x >> 4) & 1;
-    auto b = [&](int j) { return add4(add4(v[j * 16 + x], v[(j + 8) * 16 + x]), add4(v[(j + 4) * 16 + x], v[(j + 12) * 16 + x])); };
-    float4 s = add4(b(h), b(h + 2));
-#pragma unroll
-    for (int k = 16; k > 0; k >>= 1) s = add4(s, shfl_down4(s, k));
-    return s;
-}
 // cg_init.comp over this block's `count` active level-0 tiles (at(k, t): the k-th's scene, its tile
 // in t): r = b - A x (the FP32 operator) and the tile's sum of b.b in the partials' second half. A
 // cell's loads are all issued before the first is used, and one warp adds up a tile's products
@@ -351,7 +342,7 @@ DEV void residual_pass(int count, float4* sums, At&& at) {
         buf[threadIdx.x] = a4;
         __syncthreads();
         if (threadIdx.x >= 7 * 32) {
-            const float4 v = tile_tree4(buf);
+            const float4 v = warp_tree(buf);
             if (threadIdx.x == 7 * 32) M::part(d)[d.nwg + t] = v;
         }
     }

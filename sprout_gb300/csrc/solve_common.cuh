@@ -304,6 +304,17 @@ DEV void block_tree(T* buf) {
     __syncthreads();
 }
 
+// The same tree over 256 float4 by one warp: the tree's row steps of a 16-wide column by its two
+// lanes, then the column steps by shuffles; the sum comes out in lane 0.
+DEV float4 warp_tree(const float4* v) {
+    const int x = threadIdx.x & 15, h = (threadIdx.x >> 4) & 1;
+    auto b = [&](int j) { return add4(add4(v[j * 16 + x], v[(j + 8) * 16 + x]), add4(v[(j + 4) * 16 + x], v[(j + 12) * 16 + x])); };
+    float4 s = add4(b(h), b(h + 2));
+#pragma unroll
+    for (int k = 16; k > 0; k >>= 1) s = add4(s, shfl_down4(s, k));
+    return s;
+}
+
 // total() of reduce_tail.glsl:28-41: thread t sums partials t, t + 256, ... in order,
 // then the tree. Every block calls it and gets the same value.
 template <class T>

@@ -480,6 +480,17 @@ struct VSolve {
         __syncthreads();
     }
 
+    // ... where at least a block barrier lies between two calls: one warp adds up while the others go
+    // on (a tree of the whole block, seven barriers, was 5 % of an update's or way up's tile)
+    DEV void tile_sum_behind(float4 acc, int half, uint32_t slot) const {
+        s.buf[threadIdx.x] = acc;
+        __syncthreads();
+        if (threadIdx.x >= NT - 32) {
+            const float4 v = warp_tree(s.buf);
+            if (threadIdx.x == NT - 32) d.partials[half * n + slot] = v;
+        }
+    }
+
     // the compact list of active tiles of level l (one block)
     DEV void build_list(int l) const {
         const Lv L = lev(d.lv, l);
@@ -818,7 +829,7 @@ struct VSolve {
             d.vaz[i] = az;
             acc = make_float4(dot2(g.sr[k], z), dot2(z, az), dot2(z, qi), 0.0f);
         }
-        tile_sum(acc, half, tt);
+        tile_sum_behind(acc, half, tt);
     }
     DEV void mgz(const float2* rn, const float2* qn, int half) const {
         pipe(
@@ -876,7 +887,7 @@ struct VSolve {
             rn[i] = r;
             acc = make_float4(0.0f, dot2(r, r), dot2(p, q), 0.0f);
         }
-        tile_sum(acc, half, tt);
+        tile_sum_behind(acc, half, tt);
     }
     DEV void mgu(const float2* ro, const float2* qo, float2* rn, float2* qn, int half) const {
         pipe(
