@@ -459,4 +459,15 @@ DEV void report_max(uint32_t* slot, float m) {
     if (b > seen) atomicMax(slot, b);
 }
 
+// The same for a word of flags that a kernel only adds to: the warp's bits, or-ed in where this SM
+// has not seen them all (k_grid_prep on 1600 x 900 cells, mostly air: 55 us with an atomic a warp
+// on the one word, 38 now).
+DEV void report_bits(uint32_t* word, uint32_t bits) {
+    bits = __reduce_or_sync(0xffffffffu, bits);
+    if ((threadIdx.x & 31) != 0 || bits == 0u) return;
+    uint32_t seen;
+    asm volatile("ld.global.ca.u32 %0, [%1];" : "=r"(seen) : "l"(word));
+    if (bits & ~seen) atomicOr(word, bits);
+}
+
 }  // namespace sprout

@@ -227,8 +227,7 @@ __global__ void __launch_bounds__(256) k_grid_prep(DevScene d) {
         }
         if (level <= 0.0f) d.pres[i] = make_float2(0.0f, 0.0f);
     }
-    air_bits = __reduce_or_sync(0xffffffffu, air_bits);
-    if ((threadIdx.x & 31) == 0 && air_bits != 0u) atomicOr(&d.S->region_air, air_bits);
+    report_bits(&d.S->region_air, air_bits);
 }
 
 DEV void coef_face(float4 a, float4 b, float open, float& g, float& rho) {

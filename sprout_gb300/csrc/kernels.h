@@ -20,6 +20,7 @@ struct LaunchCfg {
     bool magnet = false;      // a magnet and a susceptible liquid: magnet.comp runs
     bool xtra = false;        // families, several phase groups, settling or currents: the particle pass's full form
     bool groups = false;      // phase groups past the second: their indicators are smoothed too
+    bool one_group = false;   // no phase group but the first
     int visc_mode = 0;        // 0 none, 1 explicit, 2 implicit
     bool twice = false;       // implicit viscosity between two pressure solves
     bool viscous_warm = false;   // the first solve starts from last substep's P1 (cg_scale mode 1)
