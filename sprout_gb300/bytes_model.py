@@ -23,15 +23,14 @@ def cell_bytes(stage: str, stride: int, thermal: bool, visc_mode: int) -> int:
         return 4 + 4 * stride                                  # start (row ranges), accumulators written once
     if stage == "grid":
         prep = 4 * stride + 16 + 16 + 8 + 16 + 16 + 16 + (32 if thermal else 0) + 8
-        coef_smooth = 16 + 16 + 16 + 8 + 16
-        curv = 8 + 16 + 4 + 8 + 16
+        surface = 16 + 16 + 16 + 16 + 4 + 16 + 16             # cell, comp, solid, sprop, sdf; coef, surf
         apply = 16 + 16 + 16 + 16 + 8
         heat = (16 * 5 + 8 + 4) if thermal else 0
         visc = (16 + 16 + 16 + 16 + 16 + 16 + 8) if visc_mode == 1 else 0
         if visc_mode == 2:   # visc_setup, split, diag with the level-0 matrix, coarse builds
             visc = (16 + 16 + 16 + 16 + 16) + (16 + 16 + 16 + 8) + (16 + 16 + 8 + 8 + 16 + 16 + 8 + 16) + 20
         rhs = 16 + 16 + 16 + 16 + 8 + 16 + 4 + 8 + 16 + 4 + 16
-        return prep + coef_smooth + curv + apply + heat + visc + rhs
+        return prep + surface + apply + heat + visc + rhs
     if stage == "project":
         return 16 + 16 + 8 + 16 + 8 + 4 + 4 + 16
     raise KeyError(stage)
