@@ -170,7 +170,10 @@ struct SolveState {
     uint32_t rec[3], cap[3], f_it[3], f_un[3];
     // failure injection for tests (0: off): block dbg_block arrives dbg_stall_ns late at every
     // grid barrier, and a wait gives up after dbg_spin_limit polls instead of SPIN_LIMIT
-    uint32_t dbg_block, dbg_stall_ns, dbg_spin_limit, pad3;
+    uint32_t dbg_block, dbg_stall_ns, dbg_spin_limit;
+    // whose hierarchy the coarse tile flags (ptile) describe: HIER_PLAIN, HIER_MIXED, or neither
+    // (0, after a reset): the next build in another precision writes every tile
+    uint32_t hier;
 };
 // The iterations a frame records for a solve from its recorded count (mod.rs:2569, 2603-2606):
 // rounded up to even, and the viscosity solve's to a multiple of 4 with the Jacobi
@@ -188,6 +191,8 @@ SP_HOST_DEVICE inline uint32_t recorded_limit(uint32_t rec, bool viscosity, bool
 // SolveState::error bits: a bounded wait ran out; a solve's residual or right-hand side was
 // not finite (the solve stopped)
 constexpr uint32_t ERR_TIMEOUT = 1u, ERR_DIVERGED = 2u;
+// SolveState::hier
+constexpr uint32_t HIER_PLAIN = 1u, HIER_MIXED = 2u;
 
 // The multigrid hierarchy (Levels, src/sim/mod.rs:714-753).
 struct Levels {

@@ -50,6 +50,7 @@ __constant__ int NBY[4] = {0, 0, -1, 1};
 
 struct Plain {
     static constexpr bool kMixed = false;
+    static constexpr uint32_t kHier = HIER_PLAIN;
     using acc = float;
     using acc4 = float4;
     DEV static float4 A(const DevScene& d, int i) { return d.mga[i]; }
@@ -95,6 +96,7 @@ DEV float2 unpack(uint32_t u) { return __bfloat1622float2(*reinterpret_cast<cons
 
 struct Mixed {
     static constexpr bool kMixed = true;
+    static constexpr uint32_t kHier = HIER_MIXED;
     using acc = double;
     // the dot products' partial sums and totals in FP32 as the plain solve takes them (the
     // reference's trees), widened to FP64 for the step lengths and the convergence test
@@ -257,12 +259,15 @@ DEV void galerkin(Dg&& dg, Row&& row, float& D, float4& A) {
 
 // mg_build.comp on tile t of coarse level l + 1, from level l. One tile is two latencies, its flags'
 // and its cells' (galerkin); the three levels of a 384 x 216 tank took 6, 6 and 5 us, 2.9, 2.3 and 2.1 now.
+// A tile without unknowns is cleared when its flag falls, or when the flags are the other precision's:
+// that one's builds did not clear this hierarchy.
 template <class M>
 DEV void mg_build_tile(const DevScene& d, int l, int t) {
     const Lv F = lev(d.lv, l), C = lev(d.lv, l + 1);
     const int tfx = tiles_x(F), tfy = tiles_y(F), tcx = tiles_x(C);
     const int ty = qdiv(t, C.tm), tx = t - ty * tcx;
-    const uint32_t slot = (uint32_t)C.toff + (uint32_t)t, was = d.ptile[slot];
+    const uint32_t slot = (uint32_t)C.toff + (uint32_t)t;
+    const uint32_t was = d.ptile[slot] | (d.K->hier != M::kHier ? 1u : 0u);
     uint32_t on = 0u;
 #pragma unroll
     for (int k = 0; k < 4; k++) {
@@ -1624,6 +1629,7 @@ __global__ void __launch_bounds__(NT, 2) k_mgpcg(const __grid_constant__ DevScen
             for (int t = blockIdx.x; t < T; t += gridDim.x) mg_build_tile<M>(d, l - 1, t);
         }
         if (!grid_sync(d.K)) return;
+        if (blockIdx.x == 0 && threadIdx.x == 0) d.K->hier = M::kHier;
     }
     // the active-tile lists (ptile is final now) and the inactive tiles' zero partial sums
     for (int l = blockIdx.x; l < d.lv.tail; l += gridDim.x) build_plist(d, l);   // a level a block
@@ -1803,6 +1809,7 @@ __global__ void __launch_bounds__(NT, 2) k_mgpcg_batch(BatchView B, int second) 
             for_tiles(B, l, [&](int s, const DevScene& d, int t) { mg_build_tile<M>(d, l - 1, t); });
         }
         if (!grid_sync(BK)) return;
+        for (int s = blockIdx.x * NT + threadIdx.x; s < B.ns; s += gridDim.x * NT) B.scenes[s].K->hier = M::kHier;
     }
     // every scene's active-tile lists (a block each level) and the inactive tiles' zero partials
     for (int g = blockIdx.x; g < B.ns * B.max_tail; g += gridDim.x) {
@@ -2232,6 +2239,7 @@ __global__ void k_static_prep(DevScene d, const float4* mga, const float* mgd, c
         unsigned char* k = reinterpret_cast<unsigned char*>(K);
         for (size_t b = 0; b < sizeof(SolveState); b++) k[b] = 0;
         K->cap[0] = K->cap[1] = max_iters;   // the caller's limit, not a recorded count
+        K->hier = HIER_PLAIN;                // (cleared above, as the flags say)
     }
 }
 
