@@ -406,13 +406,22 @@ DEV Tail tail_at(unsigned char* smem, float2* r, int base, int T, int nf, int nl
 }
 
 // The persistent kernels' dynamic shared memory: the level passes' exchange of cell values
-// (TileSmem), whose bytes hold the tail's right-hand sides in the tail phase (no tile is being
-// computed then), and one scene's tail.
+// (TileSmem), and one scene's tail. While no tile is being computed its bytes hold the tail's
+// right-hand sides (the tail phase) or the block's tree buffer (the totals, the refinement's checks
+// and the closing residual).
+//
+// With every array of its own a block took 119.5 KB at 1600 x 900 (a tail of 50 x 29 and coarser
+// cells), of which an SM holds one, and 304 blocks became 152; sharing the stages' bytes it is 112 KB
+// there and at most 115 with any tail of up to 2050 cells, two an SM. (A tail has more only on a grid
+// several times as long as it is wide.) A substep of the 1600 x 900 dam 1.303 -> 1.249 ms, of the mixed
+// pour on 701 x 397 2.69 -> 2.58; 8 tanks of 400 x 225 in a mixed batch 1.324 -> 1.225 (plain 1.177 ->
+// 1.102). A tank with few active tiles does not need the second block: a quarter-full dam of 800 x 450
+// takes 0.695 ms with it and 0.685 without, a full pour there 3.0 and 3.1.
+constexpr size_t kStageBytes = 17200;
 struct TileSmem {
-    unsigned char stage[2][17408];   // two tiles' fields, staged asynchronously (LevelStage, ApplyStage)
+    unsigned char stage[2][kStageBytes];   // two tiles' fields, staged asynchronously (LevelStage, ApplyStage)
     float4 red[200];         // per red slot of a way down: its right-hand side, diagonal and reciprocal
     float2 black[200];       // per black slot: its new value
-    float2 prod[NT];         // per cell: its two products of the tile's sums
 };
 constexpr size_t kTileBytes = sizeof(TileSmem);
 static_assert(kTileBytes % 16 == 0, "the tail follows");
@@ -668,13 +677,15 @@ DEV float2 sum4(float2 r, float2 t0, float2 t1, float2 t2, float2 t3) {
     return s;
 }
 
-// The tree of reduce.glsl:5-14 over a tile's 256 products (cell ly * 16 + lx), by one warp: the
-// tree's row steps of a column by its two lanes, then the column steps by shuffles; the sum
-// comes out in lane 0.
-DEV float2 tile_tree(const float2* v) {
+// The tree of reduce.glsl:5-14 over a tile's 256 products (a cell's at the number of the thread that
+// has it in the smoothing passes: product_of), by one warp: the tree's row steps of a column by its
+// two lanes, then the column steps by shuffles; the sum comes out in lane 0.
+DEV int product_of(int lx, int ly) { return ((lx + ly) & 1 ? 0 : 128) + ly * 8 + (lx >> 1); }
+DEV float2 tile_tree(const float2* prod) {
     const int x = threadIdx.x & 15, h = (threadIdx.x >> 4) & 1;
+    const float2* const v = prod + product_of(x, h) - h * 8;   // (rows of one parity: one colour a lane)
     auto b = [&](int j) {
-        const float2 v0 = v[j * 16 + x], v1 = v[(j + 4) * 16 + x], v2 = v[(j + 8) * 16 + x], v3 = v[(j + 12) * 16 + x];
+        const float2 v0 = v[j * 8], v1 = v[(j + 4) * 8], v2 = v[(j + 8) * 8], v3 = v[(j + 12) * 8];
         return make_float2((v0.x + v2.x) + (v1.x + v3.x), (v0.y + v2.y) + (v1.y + v3.y));
     };
     const float2 b0 = b(h), b1 = b(h + 2);
@@ -689,14 +700,15 @@ DEV float2 tile_tree(const float2* v) {
 constexpr int kTreeWarp = 7;
 
 // A tile's fields as they are staged: thread t's own cell in entry t, its cell of the ring in
-// entry t - 128 of the e arrays.
+// entry t - 128 of the e arrays. On level 0 p's entries take the products of the tile's sums once
+// the way down has read its direction there (the way up stages nothing in them).
 template <class M>
 struct LevelStage {
     typename M::Row a[NT], ea[32];
     float2 r[NT], er[98], q[NT], eq[98], p[NT], x[NT];
     typename M::Diag y[NT], ey[98];
 };
-static_assert(sizeof(LevelStage<Plain>) <= sizeof(TileSmem::stage) / 2, "two tiles' fields");
+static_assert(sizeof(LevelStage<Plain>) == kStageBytes && sizeof(LevelStage<Mixed>) <= kStageBytes, "two tiles' fields");
 struct ApplyStage {
     float4 a[NT];
     float2 z[NT], o[NT], ez[64], eo[64];
@@ -768,7 +780,7 @@ DEV bool down_pass_(const Geo& g, int count, bool top, Of&& of, At&& at, Next&& 
         }
         cp_commit();
         cp_wait<1>();
-        const Stage& n = stage(turn);
+        Stage& n = stage(turn);
         const int2 og = tile_origin(cur.F, cur.t);
         const bool fused = cur.a.q != nullptr, in = og.x + g.lx < cur.F.w && og.y + g.ly < cur.F.h;
         const int i = l_at(cur.F, og.x + g.lx, og.y + g.ly);
@@ -794,7 +806,7 @@ DEV bool down_pass_(const Geo& g, int count, bool top, Of&& of, At&& at, Next&& 
             }
         }
         const bool unk = M::unk(y), eunk = M::unk(ey);
-        if (top) S.prod[g.ly * 16 + g.lx] = f2sel(unk, make_float2(r.x * r.x, r.y * r.y), 0.0f);
+        if (top) n.p[t] = f2sel(unk, make_float2(r.x * r.x, r.y * r.y), 0.0f);
         r = f2sel(unk, r, -0.0f);
         er = f2sel(eunk, er, -0.0f);
         if (g.red) {
@@ -825,7 +837,7 @@ DEV bool down_pass_(const Geo& g, int count, bool top, Of&& of, At&& at, Next&& 
             S.black[s] = z;
             if (own && in) of(cur.scene).mgx[i] = z;
         } else if (top && t >= 32 * kTreeWarp) {
-            const float2 rr = tile_tree(S.prod);
+            const float2 rr = tile_tree(n.p);
             if ((t & 31) == 0) reinterpret_cast<float2*>(M::part(of(cur.scene)) + cur.t)[1] = rr;
         }
         __syncthreads();
@@ -876,7 +888,7 @@ DEV bool up_pass_(const Geo& g, int count, bool top, Of&& of, At&& at, Next&& ne
     float2* const sred = reinterpret_cast<float2*>(S.red);
     const int t = threadIdx.x;
     bool bad = false;
-    using Stage = LevelStage<M>;   // (q: the pre-smoothed values, p and x: the coarse values of the tile and the ring)
+    using Stage = LevelStage<M>;   // (q: the red cells' pre-smoothed values, then their coarse ones; x: the ring's coarse ones)
     auto fetch = [&](const UpTile& T, Stage& n) {
         const DevScene& d = of(T.scene);
         const int2 og = tile_origin(T.F, T.t);
@@ -887,8 +899,8 @@ DEV bool up_pass_(const Geo& g, int count, bool top, Of&& of, At&& at, Next&& ne
         cp_async<sizeof(typename M::Diag)>(&n.y[t], M::diags(d) + i, in);
         cp_async<8>(&n.r[t], T.r + i, in);
         if (g.red) {
-            cp_async<8>(&n.q[t], d.mgx + i, in);
-            if (!T.zs) cp_async<8>(&n.p[t], T.zc + (in ? (y >> 1) * T.C.w + (x >> 1) : 0), in);
+            cp_async<8>(&n.q[t - 128], d.mgx + i, in);
+            if (!T.zs) cp_async<8>(&n.q[t], T.zc + (in ? (y >> 1) * T.C.w + (x >> 1) : 0), in);
         }
         if (g.kind != 0) {
             const int ex = og.x + g.ex, ey = og.y + g.ey;
@@ -910,9 +922,9 @@ DEV bool up_pass_(const Geo& g, int count, bool top, Of&& of, At&& at, Next&& ne
         return M::template quot<SLOW>(s, y);
     };
     auto corrected = [](float2 v, float2 zc) { return make_float2(v.x + MG_OMEGA * zc.x, v.y + MG_OMEGA * zc.y); };
-    auto tree = [&](const UpTile& T) {
+    auto tree = [&](const UpTile& T, const float2* prod) {
         if (t < 32 * kTreeWarp) return;
-        const float2 rz = tile_tree(S.prod);
+        const float2 rz = tile_tree(prod);
         if ((t & 31) == 0) reinterpret_cast<float2*>(M::part(of(T.scene)) + T.t)[0] = rz;
     };
     auto stage = [](int turn) -> Stage& { return *reinterpret_cast<Stage*>(dyn_smem + (turn & 1) * sizeof(TileSmem::stage) / 2); };
@@ -931,9 +943,9 @@ DEV bool up_pass_(const Geo& g, int count, bool top, Of&& of, At&& at, Next&& ne
         }
         cp_commit();
         cp_wait<1>();
-        const Stage& n = stage(turn);
+        Stage& n = stage(turn);
         const int2 og = tile_origin(cur.F, cur.t);
-        const int X = og.x + g.lx, Y = og.y + g.ly, i = l_at(cur.F, X, Y), cell = g.ly * 16 + g.lx;
+        const int X = og.x + g.lx, Y = og.y + g.ly, i = l_at(cur.F, X, Y);
         const bool in = X < cur.F.w && Y < cur.F.h;
         const typename M::Diag y = n.y[t];
         typename M::Diag ey = M::no_diag();
@@ -943,8 +955,8 @@ DEV bool up_pass_(const Geo& g, int count, bool top, Of&& of, At&& at, Next&& ne
         if (g.red) {
             // (the tail's values are this block's own, in shared memory)
             float2 zc = make_float2(0.0f, 0.0f);
-            if (unk) zc = cur.zs ? cur.zs[(Y >> 1) * cur.C.w + (X >> 1)] : n.p[t];
-            sred[g.s] = f2sel(unk, corrected(n.q[t], zc), -0.0f);
+            if (unk) zc = cur.zs ? cur.zs[(Y >> 1) * cur.C.w + (X >> 1)] : n.q[t];
+            sred[g.s] = f2sel(unk, corrected(n.q[t - 128], zc), -0.0f);
             if (g.kind == 2) {
                 const int EX = og.x + g.ex, EY = og.y + g.ey;
                 float2 ez = make_float2(0.0f, 0.0f);
@@ -964,7 +976,7 @@ DEV bool up_pass_(const Geo& g, int count, bool top, Of&& of, At&& at, Next&& ne
             S.black[s] = f2sel(u, z, -0.0f);
             if (own) {
                 if (in) of(cur.scene).mgz[i] = f2sel(u, z, 0.0f);
-                if (top) S.prod[cell] = f2sel(u, make_float2(r.x * z.x, r.y * z.y), 0.0f);
+                if (top) n.p[t] = f2sel(u, make_float2(r.x * z.x, r.y * z.y), 0.0f);
             }
         }
         __syncthreads();
@@ -973,11 +985,11 @@ DEV bool up_pass_(const Geo& g, int count, bool top, Of&& of, At&& at, Next&& ne
             const float2 z = value(sum4(r, mul2(w.x, S.black[g.s - g.e]), mul2(w.y, S.black[g.s - g.e + 1]), mul2(w.z, S.black[g.s - SP]),
                                         mul2(w.w, S.black[g.s + SP])), y);
             if (in) of(cur.scene).mgz[i] = f2sel(unk, z, 0.0f);
-            if (top) S.prod[cell] = f2sel(unk, make_float2(r.x * z.x, r.y * z.y), 0.0f);
+            if (top) n.p[t] = f2sel(unk, make_float2(r.x * z.x, r.y * z.y), 0.0f);
         }
         if (top) {
             __syncthreads();
-            tree(cur);
+            tree(cur, n.p);
         }
         if (!more) break;
     }
@@ -1015,7 +1027,7 @@ DEV void apply_pass(int count, Of&& of, At&& at, Next&& next) {
     const int hr = t - 128, hj = t & 15;   // the halo cell of threads 128 .. 191
     const bool halo = t >= 128 && t < 192;
     const int hx = hr < 16 ? -1 : hr < 32 ? 16 : hj, hy = hr < 32 ? hj : hr < 48 ? -1 : 16;
-    const int s0 = (ly + 1) * PW + lx + 1, sh = (hy + 1) * PW + hx + 1;
+    const int s0 = (ly + 1) * PW + lx + 1, sh = (hy + 1) * PW + hx + 1, sp = product_of(lx, ly);
     using Stage = ApplyStage;
     auto nob = [](const ApplyTile& T) { return T.b0 == 0.0f && T.b1 == 0.0f; };
     auto fetch = [&](const ApplyTile& T, Stage& n) {
@@ -1044,7 +1056,8 @@ DEV void apply_pass(int count, Of&& of, At&& at, Next&& next) {
     };
     auto stage = [](int slot) -> Stage& { return *reinterpret_cast<Stage*>(dyn_smem + slot * sizeof(Stage)); };
     int slot = 0;   // this tile's stage
-    static_assert(3 * sizeof(Stage) <= sizeof(S.stage), "three tiles in flight");
+    static_assert(3 * sizeof(Stage) + NT * sizeof(float2) <= sizeof(S.stage), "three tiles in flight, and the products");
+    float2* const prod = reinterpret_cast<float2*>(dyn_smem + 3 * sizeof(Stage));
     int k = next(0);
     if (k >= count) return;
     ApplyTile T = at(k), T1 = T;
@@ -1087,10 +1100,10 @@ DEV void apply_pass(int count, Of&& of, At&& at, Next&& next) {
             cur.p_new[i] = p;
             of(cur.scene).cgq[i] = q;
         }
-        S.prod[t] = f2sel(D > 0.0f, make_float2(p.x * q.x, p.y * q.y), 0.0f);
+        prod[sp] = f2sel(D > 0.0f, make_float2(p.x * q.x, p.y * q.y), 0.0f);
         __syncthreads();
         if (t >= 32 * kTreeWarp) {
-            const float2 pq = tile_tree(S.prod);
+            const float2 pq = tile_tree(prod);
             if ((t & 31) == 0) reinterpret_cast<float2*>(M::part(of(cur.scene)) + of(cur.scene).nwg + cur.t)[1] = pq;
         }
         if (!more) break;
@@ -1611,10 +1624,9 @@ __global__ void __launch_bounds__(NT, 2) k_mgpcg(const __grid_constant__ DevScen
     using acc = typename M::acc;
     using acc4 = typename M::acc4;
     __shared__ TileCache tc;
-    // the block's tree buffer: float pairs in mixed precision (the refinement's checks), whose
-    // bytes the dot products' trees use as acc4 in other phases
-    __shared__ typename std::conditional<M::kMixed, FF4, acc4>::type buf_raw[NT];
-    acc4* buf = reinterpret_cast<acc4*>(buf_raw);
+    // the block's tree buffer, in the stages' bytes: no tile is staged while it is used
+    static_assert(NT * sizeof(FF4) <= sizeof(TileSmem::stage), "the refinement's checks sum float pairs");
+    acc4* const buf = reinterpret_cast<acc4*>(dyn_smem);
     __shared__ Solve<acc> K;
     const DevParams* P = d.P;
     const int n = d.nwg;
@@ -1662,9 +1674,9 @@ __global__ void __launch_bounds__(NT, 2) k_mgpcg(const __grid_constant__ DevScen
                 // the apply phase rewrites it, and the partials' second half until it sums p.q
                 if (it > 1 && want_check(K)) {
                     FF4* pc = reinterpret_cast<FF4*>(d.partials64) + n;
-                    for_active(d, 0, tc, [&](int t) { check_tile(d, t, d.cgq, pc, reinterpret_cast<FF4*>(buf_raw)); });
+                    for_active(d, 0, tc, [&](int t) { check_tile(d, t, d.cgq, pc, reinterpret_cast<FF4*>(dyn_smem)); });
                     if (!grid_sync(d.K)) return;
-                    const Dbl4 tot = to_dbl(total(pc, n, reinterpret_cast<FF4*>(buf_raw)));
+                    const Dbl4 tot = to_dbl(total(pc, n, reinterpret_cast<FF4*>(dyn_smem)));
                     __shared__ int s_adopt;
                     if (threadIdx.x == 0) s_adopt = decide_check(K, tot) ? 1 : 0;
                     __syncthreads();
@@ -1700,9 +1712,9 @@ __global__ void __launch_bounds__(NT, 2) k_mgpcg(const __grid_constant__ DevScen
     double true_rel = -1.0;
     if constexpr (M::kMixed) {
         FF4* pt = reinterpret_cast<FF4*>(d.partials64);
-        for_active(d, 0, tc, [&](int t) { true_residual_tile(d, t, pt, reinterpret_cast<FF4*>(buf_raw)); });
+        for_active(d, 0, tc, [&](int t) { true_residual_tile(d, t, pt, reinterpret_cast<FF4*>(dyn_smem)); });
         if (!grid_sync(d.K)) return;
-        const Dbl4 t4 = to_dbl(total(pt, n, reinterpret_cast<FF4*>(buf_raw)));
+        const Dbl4 t4 = to_dbl(total(pt, n, reinterpret_cast<FF4*>(dyn_smem)));
         true_rel = t4.y > 0.0 ? sqrt(t4.x / t4.y) : 0.0;
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) scal_stats<M, acc>(d.K, K, second, true_rel);
@@ -1789,10 +1801,9 @@ __global__ void __launch_bounds__(NT, 2) k_mgpcg_batch(BatchView B, int second) 
     using acc = typename M::acc;
     using acc4 = typename M::acc4;
     __shared__ TileCache tc;
-    // the block's tree buffer: float pairs in mixed precision (the refinement's checks), whose
-    // bytes the dot products' trees use as acc4 in other phases
-    __shared__ typename std::conditional<M::kMixed, FF4, acc4>::type buf_raw[NT];
-    acc4* buf = reinterpret_cast<acc4*>(buf_raw);
+    // the block's tree buffer, in the stages' bytes: no tile is staged while it is used
+    static_assert(NT * sizeof(FF4) <= sizeof(TileSmem::stage), "the refinement's checks sum float pairs");
+    acc4* const buf = reinterpret_cast<acc4*>(dyn_smem);
     __shared__ int s_run;
     Solve<acc>* KS = reinterpret_cast<Solve<acc>*>(B.scal);
     SolveState* BK = B.K;
@@ -1947,14 +1958,14 @@ __global__ void __launch_bounds__(NT, 2) k_mgpcg_batch(BatchView B, int second) 
             __syncthreads();
             if (s_run) {
                 for_active_b(B, 0, tc, [&](int s, const DevScene& d, int t) {
-                    if (chk(s)) check_tile(d, t, d.cgq, reinterpret_cast<FF4*>(d.partials64) + d.nwg, reinterpret_cast<FF4*>(buf_raw));
+                    if (chk(s)) check_tile(d, t, d.cgq, reinterpret_cast<FF4*>(d.partials64) + d.nwg, reinterpret_cast<FF4*>(dyn_smem));
                 });
                 if (!grid_sync(BK)) return;
                 // each scene's decision by one block (it alone writes KS[s] until the next barrier)
                 for (int s = blockIdx.x; s < B.ns; s += gridDim.x) {
                     if (!chk(s)) continue;
                     const DevScene& d = B.scenes[s];
-                    const Dbl4 tot = to_dbl(total(reinterpret_cast<FF4*>(d.partials64) + d.nwg, d.nwg, reinterpret_cast<FF4*>(buf_raw)));
+                    const Dbl4 tot = to_dbl(total(reinterpret_cast<FF4*>(d.partials64) + d.nwg, d.nwg, reinterpret_cast<FF4*>(dyn_smem)));
                     if (threadIdx.x == 0) KS[s].adopt = decide_check(KS[s], tot) ? 1u : 0u;
                     __syncthreads();
                 }
@@ -2010,7 +2021,7 @@ __global__ void __launch_bounds__(NT, 2) k_mgpcg_batch(BatchView B, int second) 
     }
     if constexpr (M::kMixed) {
         for_active_b(B, 0, tc, [&](int s, const DevScene& d, int t) {
-            true_residual_tile(d, t, reinterpret_cast<FF4*>(d.partials64), reinterpret_cast<FF4*>(buf_raw));
+            true_residual_tile(d, t, reinterpret_cast<FF4*>(d.partials64), reinterpret_cast<FF4*>(dyn_smem));
         });
         if (!grid_sync(BK)) return;
     }
@@ -2018,7 +2029,7 @@ __global__ void __launch_bounds__(NT, 2) k_mgpcg_batch(BatchView B, int second) 
         const DevScene& d = B.scenes[s];
         double true_rel = -1.0;
         if constexpr (M::kMixed) {
-            const Dbl4 t4 = to_dbl(total(reinterpret_cast<FF4*>(d.partials64), d.nwg, reinterpret_cast<FF4*>(buf_raw)));
+            const Dbl4 t4 = to_dbl(total(reinterpret_cast<FF4*>(d.partials64), d.nwg, reinterpret_cast<FF4*>(dyn_smem)));
             true_rel = t4.y > 0.0 ? sqrt(t4.x / t4.y) : 0.0;
         }
         if (threadIdx.x == 0) scal_stats<M, acc>(d.K, KS[s], second, true_rel);
