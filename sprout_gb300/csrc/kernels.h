@@ -11,6 +11,7 @@ namespace sprout {
 // What the host decided for this configuration of the tank.
 struct LaunchCfg {
     uint32_t n_slots = 0;
+    int sms = 1;              // the device's multiprocessors
     bool thermal = false;
     bool heat = false;        // thermal and heat_rate > 0: heat.comp runs
     bool rheo = false;        // a non-Newtonian liquid is in the tank: rheo.comp runs

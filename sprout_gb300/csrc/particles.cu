@@ -1050,15 +1050,16 @@ void launch_sort(const DevScene& d, const LaunchCfg& cfg, cudaStream_t st) {
 }
 
 void launch_p2g(const DevScene& d, const LaunchCfg& cfg, cudaStream_t st) {
-    (void)cfg;
     dim3 tiles((d.W + P2G_T - 1) / P2G_T, (d.H + P2G_T - 1) / P2G_T);
     size_t smem = (size_t)P2G_T * P2G_T * (d.stride + 1) * sizeof(int);
-    // Few tiles, and of those only some with liquid, leave most SMs one block: more threads then
-    // hide the latency of its chains of shared atomics (384 x 216, 336 tiles: 22.6 us with 256
-    // threads, 16.6 with 512; 128 x 72: 22.0 and 15.8). With four tiles an SM or more the blocks
-    // hide each other's, and fewer threads wait at the tile's ends (512 x 288, 576 tiles: 28.7 and
-    // 30.7; 1600 x 900: 72 and 86).
-    const bool few = tiles.x * tiles.y <= 3 * 152;
+    // 512 threads a tile hide the latency of its chains of shared atomics, while the tiles with liquid
+    // (a tile of 256 cells at the usual four particles each holds 1024) fit on the device at once, two
+    // blocks an SM; past that 256 threads, whose four blocks an SM hide each other's, until both are
+    // bound by the atomics' rate. By tiles with liquid (152 SMs: the line at 304), 256 against 512
+    // threads in us: 138 (512 x 288 dam) 25.2 / 20.7; 186 24.7 / 20.9; 298 (384 x 216 full of eight
+    // liquids) 30.2 / 28.6; 304 (768 x 432 dam) 35.0 / 30.9; 324 31.7 / 35.0; 351 32.6 / 35.0; 410
+    // 33.0 / 39.0; 541 41.0 / 41.1; 856 65.0 / 59.6; 1336 (1600 x 900 dam) 85 / 100.
+    const bool few = cfg.n_slots <= 2u * 1024u * (uint32_t)cfg.sms;
     k_p2g<<<tiles, few ? 512 : 256, smem, st>>>(d);
 }
 

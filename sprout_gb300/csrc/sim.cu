@@ -295,6 +295,7 @@ struct SproutSim {
         CUDA_TRY(cudaMemset(d.rl, 0xff, nc * sizeof(int2)));   // no cell rigid before the first rigid pass
         std::vector<float> nt(nc, NO_TEMP);
         CUDA_TRY(cudaMemcpy(solid_t, nt.data(), nc * sizeof(float), cudaMemcpyHostToDevice));
+        CUDA_TRY(cudaDeviceGetAttribute(&cfg.sms, cudaDevAttrMultiProcessorCount, device));
         tuned = tuned_launch(W, H);
         mg_max = pressure_blocks_max(device, pressure_smem(d.lv), false);
         cfg.mg_blocks = pick_blocks(launch_req.pressure_blocks, mg_max, tuned.pressure_blocks);
