@@ -21,7 +21,6 @@ struct LaunchCfg {
     bool magnet = false;      // a magnet and a susceptible liquid: magnet.comp runs
     bool xtra = false;        // families, several phase groups, settling or currents: the particle pass's full form
     bool groups = false;      // phase groups past the second: their indicators are smoothed too
-    bool one_group = false;   // no phase group but the first
     int visc_mode = 0;        // 0 none, 1 explicit, 2 implicit
     bool twice = false;       // implicit viscosity between two pressure solves
     bool viscous_warm = false;   // the first solve starts from last substep's P1 (cg_scale mode 1)
@@ -29,7 +28,6 @@ struct LaunchCfg {
     int visc_sweeps = 2;      // Gauss-Seidel sweeps per visit of a level (1 or 2)
     int visc_blocks = 0;      // blocks of the persistent viscosity kernel
     int mg_blocks = 0;        // blocks of the persistent pressure kernel
-    int mg_threads = 256;
     bool mixed = false;       // the mixed-precision pressure solve
     int mg_blocks_mixed = 0;  // blocks of its persistent kernel
 };
@@ -236,8 +234,8 @@ cudaError_t rasterize_device(const Scene& sc, float* sdf, float4* solid, uint32_
 // Blocks of the persistent pressure kernel (plain or mixed precision) that fit on the
 // device at once.
 int pressure_blocks_max(int device, size_t smem, bool mixed);
-// Dynamic shared memory of the persistent pressure kernel: the tail levels of each block.
+// Dynamic shared memory of a block of the persistent pressure kernels, single and batched: the tiles in
+// flight and the tail levels.
 size_t pressure_smem(const Levels& lv);
-// ... and of the batched one, whose staging regions share it with the tail.
 
 }  // namespace sprout

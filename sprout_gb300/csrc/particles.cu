@@ -688,8 +688,7 @@ __global__ void __launch_bounds__(256) k_advance(DevScene d) {
 
 constexpr int SCAN_BLOCK = 1024, SCAN_SPAN = 4 * SCAN_BLOCK;   // threads of a block, counts it scans
 
-// Block-wise exclusive scan of count[0..n) into start, block totals into tmp.
-// the exclusive sum of the block's x in thread order; *total: of all of them
+// The exclusive sum of the block's x in thread order; *total: of all of them
 DEV uint32_t scan_exclusive(uint32_t x0, uint32_t* warp_sums, uint32_t* total) {
     uint32_t x = x0;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -714,10 +713,10 @@ DEV uint32_t scan_exclusive(uint32_t x0, uint32_t* warp_sums, uint32_t* total) {
     return (wid > 0 ? warp_sums[wid - 1] : 0u) + x - x0;
 }
 
-// The scan in two kernels: each block's own exclusive sums and its total, then to each block the
-// sum of the totals before it, which it adds up itself (four counts a thread keep those few: 352
-// at 1600 x 900, one a thread at 4 million cells). The totals scanned by a kernel of their
-// own were one more node of the chain, 4 us of a substep.
+// The exclusive scan of count[0 .. n) into start in two kernels: each block's own sums, and its total
+// into tmp; then to each block the sum of the totals before it, which it adds up itself (four counts
+// a thread keep those few: 352 at 1600 x 900, one a thread at 4 million cells). The totals scanned
+// by a kernel of their own were one more node of the chain, 4 us of a substep.
 __global__ void __launch_bounds__(SCAN_BLOCK) k_scan_blocks(const uint32_t* count, uint32_t* start, uint32_t* tmp, int n) {
     __shared__ uint32_t warp_sums[SCAN_BLOCK / 32];
     const int i = blockIdx.x * SCAN_SPAN + 4 * threadIdx.x;

@@ -177,11 +177,8 @@ DEV bool finite4(const A4& a) { return isfinite(a.x) && isfinite(a.y) && isfinit
 
 // ---- setup phases ---------------------------------------------------------------------
 
-// Unknowns of the V-cycle's level (M's copy of the diagonal) and of the CG operator.
-template <class M>
-DEV bool unknown(const DevScene& d, const Lv& L, int x, int y) { return l_inside(L, x, y) && M::Dg(d, l_at(L, x, y)) > 0.0f; }
+// Unknowns of the CG operator.
 DEV bool unknown_op(const DevScene& d, const Lv& L, int x, int y) { return l_inside(L, x, y) && d.mgd[l_at(L, x, y)] > 0.0f; }
-
 
 // cg_scale.comp on level-0 tile t: warm start from last substep's potential rescaled to
 // this substep. Also level 0's diagonal with its reciprocal, or (mixed) its matrix in BF16, for

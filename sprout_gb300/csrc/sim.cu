@@ -282,11 +282,10 @@ struct SproutSim {
         A(d.mgx, (size_t)d.lv.total);
         A(d.mgz, (size_t)d.lv.total);
         A(d.mgr, (size_t)d.lv.total);
-        // (one entry more: the level passes read cells in pairs)
-        A(d.mgr2, nc + 1);
-        A(d.cgp, nc + 1);
-        A(d.cgp2, nc + 1);
-        A(d.cgq, nc + 1);
+        A(d.mgr2, nc);
+        A(d.cgp, nc);
+        A(d.cgp2, nc);
+        A(d.cgq, nc);
         A(d.ptile, (size_t)d.lv.tiles);
         A(d.plist, (size_t)d.lv.tiles);
         A(d.pcount, (size_t)kMaxLevels);
@@ -606,7 +605,6 @@ struct SproutSim {
         want.rigid = (caps & CAP_RIGID) != 0u;
         want.xtra = tank.families > 0 || (tank.group_mask & ~1u) != 0u || !currents.empty() || tank.chan_e >= 0 || (caps & CAP_RIGID) != 0u;
         want.groups = (tank.group_mask & 12u) != 0u;
-        want.one_group = tank.group_mask == 1u;
         want.visc_mode = visc_mode;
         want.twice = visc_mode == 2 && params.viscous_projection != 0;
         want.viscous_warm = params.viscous_warm != 0;
@@ -614,7 +612,7 @@ struct SproutSim {
         want.visc_sweeps = (int)std::min(std::max(params.viscosity_mg_sweeps, 1u), 2u);
         want.visc_blocks = pick_blocks(launch_req.viscosity_blocks, visc_max[want.visc_sweeps - 1], tuned.viscosity_blocks);
         want.mixed = mixed;
-        bool same = want.n_slots == cfg.n_slots && want.thermal == cfg.thermal && want.heat == cfg.heat && want.rheo == cfg.rheo && want.settle == cfg.settle && want.magnet == cfg.magnet && want.elastic == cfg.elastic && want.rigid == cfg.rigid && want.xtra == cfg.xtra && want.groups == cfg.groups && want.one_group == cfg.one_group &&
+        bool same = want.n_slots == cfg.n_slots && want.thermal == cfg.thermal && want.heat == cfg.heat && want.rheo == cfg.rheo && want.settle == cfg.settle && want.magnet == cfg.magnet && want.elastic == cfg.elastic && want.rigid == cfg.rigid && want.xtra == cfg.xtra && want.groups == cfg.groups &&
                     want.visc_mode == cfg.visc_mode && want.twice == cfg.twice && want.viscous_warm == cfg.viscous_warm &&
                     want.visc_levels == cfg.visc_levels && want.visc_sweeps == cfg.visc_sweeps &&
                     want.visc_blocks == cfg.visc_blocks && want.mixed == cfg.mixed && d.stride == std::max(tank.stride, 8);
