@@ -81,10 +81,12 @@ struct Plain {
         r = make_float2(v.x, v.y);
         y = make_float2(v.z, v.w);
     }
-    template <bool SLOW>
-    DEV static float2 quot(float2 a, const Diag& y) { return make_float2(quot1<SLOW>(a.x, y), quot1<SLOW>(a.y, y)); }
-    // whether a may be divided by y's diagonal the fast way (an unknown's)
-    DEV static bool ok(float2 a, const Diag& y) { return value_ok(a.x) && value_ok(a.y) && y.y > 0.0f; }
+    // a / D the fast way, whether it may be taken that way (an unknown's), the IEEE division, and y
+    // with a reciprocal that says it may not
+    DEV static float2 quot(float2 a, const Diag& y) { return quot2(a, y); }
+    DEV static bool ok(float2 a, const Diag& y) { return quot_ok<60>(a, y.y); }
+    DEV static float2 quot_ieee(float2 a, const Diag& y) { return quot2_ieee(a, y); }
+    DEV static Diag spoilt(const Diag& y) { return make_float2(y.x, __int_as_float(0x7fffffff)); }
 };
 
 // a pair of BF16 values in 32 bits (x in the low half), rounded to nearest even
@@ -156,9 +158,10 @@ struct Mixed {
         r = make_float2(v.x, v.y);
         y = v.z;
     }
-    template <bool SLOW>
     DEV static float2 quot(float2 a, const Diag& y) { return make_float2(a.x * y, a.y * y); }
     DEV static bool ok(float2, const Diag&) { return true; }
+    DEV static float2 quot_ieee(float2 a, const Diag&) { return a; }   // (never taken)
+    DEV static Diag spoilt(const Diag& y) { return y; }
 };
 
 template <class T>
@@ -606,6 +609,12 @@ __device__ __noinline__ void tail_setup_of(const DevScene* d) { tail_setup<M>(*d
 // block 2.3-3.0 -> 1.7-2.0. Tried and slower: ten lanes of a warp marching up a tile without
 // block barriers (too few warps to hide its ~1000 instructions a row pair: 19 / 12 / 13 us).
 //
+// A quotient whose operands left the fast form's range is taken again by its thread with the IEEE
+// division, where it stands: few threads do, but in a tank with spray some do in most phases (small
+// drops converge to residuals below the range long before the rest). With the block's whole pass
+// taken again instead, a batch of 64 uneven dam breaks took 24 to 26.6 ms a substep once 0.3 % of its
+// tiles held such a drop, 18.8 to 19.8 now (18 to 18.8 without one); a 384 x 216 dam 0.68 and 0.48.
+//
 // The values are those of the shaders' work groups, term by term in their order. A neighbour
 // that is no unknown is a term less there; here its value is -0 (or, where the term is
 // subtracted, +0), which adds nothing to any sum.
@@ -730,12 +739,11 @@ struct DownTile {
 // takes): red-black Gauss-Seidel from zero, the residual summed over 2 x 2 cells into the next
 // level. On level 0 (top) also the tile's sums of r.r into part[tile].zw (the way up adds those
 // of r.z) and, where q is set, x += alpha p, r -= alpha q (a cell that is no unknown has p = 0,
-// and what its r holds is never used). True if an operand left the fast quotients' range.
-template <class M, bool SLOW, class Of, class At, class Next>
-DEV bool down_pass_(const Geo& g, int count, bool top, Of&& of, At&& at, Next&& next) {
+// and what its r holds is never used).
+template <class M, class Of, class At, class Next>
+DEV void down_pass(const Geo& g, int count, bool top, Of&& of, At&& at, Next&& next) {
     TileSmem& S = *reinterpret_cast<TileSmem*>(dyn_smem);
     const int t = threadIdx.x;
-    bool bad = false;
     using Stage = LevelStage<M>;
     auto fetch = [&](const DownTile& T, Stage& n) {
         const DevScene& d = of(T.scene);
@@ -763,7 +771,7 @@ DEV bool down_pass_(const Geo& g, int count, bool top, Of&& of, At&& at, Next&& 
     };
     auto stage = [](int turn) -> Stage& { return *reinterpret_cast<Stage*>(dyn_smem + (turn & 1) * sizeof(TileSmem::stage) / 2); };
     int k = next(0);
-    if (k >= count) return false;
+    if (k >= count) return;
     DownTile T = at(k);
     fetch(T, stage(0));
     cp_commit();
@@ -789,7 +797,7 @@ DEV bool down_pass_(const Geo& g, int count, bool top, Of&& of, At&& at, Next&& 
             r.x = r.x - cur.a.ax * q.x;
             r.y = r.y - cur.a.ay * q.y;
             if (in) {
-                if (!SLOW) of(cur.scene).pres[i] = make_float2(x.x + cur.a.ax * p.x, x.y + cur.a.ay * p.y);   // (once)
+                of(cur.scene).pres[i] = make_float2(x.x + cur.a.ax * p.x, x.y + cur.a.ay * p.y);
                 cur.a.r_out[i] = r;
             }
         }
@@ -807,13 +815,12 @@ DEV bool down_pass_(const Geo& g, int count, bool top, Of&& of, At&& at, Next&& 
         r = f2sel(unk, r, -0.0f);
         er = f2sel(eunk, er, -0.0f);
         if (g.red) {
-            if (!SLOW) bad |= unk && !M::ok(r, y);
-            S.red[g.s] = M::pack_red(r, y);
-            if (in) of(cur.scene).mgx[i] = f2sel(unk, M::template quot<SLOW>(r, y), 0.0f);
-            if (g.kind == 2) {
-                if (!SLOW) bad |= eunk && !M::ok(er, ey);
-                S.red[g.es] = M::pack_red(er, ey);
-            }
+            const bool odd = unk && !M::ok(r, y);
+            float2 z = M::quot(r, y);
+            if (__builtin_expect(odd, 0)) z = M::quot_ieee(r, y);
+            S.red[g.s] = M::pack_red(r, odd ? M::spoilt(y) : y);
+            if (in) of(cur.scene).mgx[i] = f2sel(unk, z, 0.0f);
+            if (g.kind == 2) S.red[g.es] = M::pack_red(er, eunk && !M::ok(er, ey) ? M::spoilt(ey) : ey);
         }
         __syncthreads();
         if (t < 160) {   // the black cells, and warp 4 those of the ring
@@ -825,12 +832,25 @@ DEV bool down_pass_(const Geo& g, int count, bool top, Of&& of, At&& at, Next&& 
                 float2 v;
                 typename M::Diag yn;
                 M::unpack_red(S.red[j], v, yn);
-                return M::template quot<SLOW>(mul2(wq, v), yn);
+                return M::quot(mul2(wq, v), yn);
             };
             const float2 sum = sum4(own ? r : er, term(w.x, s - e), term(w.y, s - e + 1), term(w.z, s - SP), term(w.w, s + SP));
             const bool u = own ? unk : eunk;
-            if (!SLOW) bad |= u && !M::ok(sum, yo);
-            const float2 z = f2sel(u, M::template quot<SLOW>(sum, yo), 0.0f);
+            float2 z = M::quot(sum, yo);
+            if (__builtin_expect(u && !M::ok(sum, yo), 0)) {   // (a spoilt neighbour's term is not a number)
+                float2 a = own ? r : er;
+#pragma unroll 1
+                for (int q = 0; q < 4; q++) {
+                    float2 v;
+                    typename M::Diag yn;
+                    M::unpack_red(S.red[q < 2 ? s - e + q : s + (2 * q - 5) * SP], v, yn);
+                    v = M::quot_ieee(mul2(wcomp(w, q), v), yn);
+                    a.x += v.x;
+                    a.y += v.y;
+                }
+                z = M::quot_ieee(a, yo);
+            }
+            z = f2sel(u, z, 0.0f);
             S.black[s] = z;
             if (own && in) of(cur.scene).mgx[i] = z;
         } else if (top && t >= 32 * kTreeWarp) {
@@ -854,18 +874,6 @@ DEV bool down_pass_(const Geo& g, int count, bool top, Of&& of, At&& at, Next&& 
         }
         if (!more) break;
     }
-    return bad;
-}
-// The tiles of a pass in which a fast quotient met an operand out of range are taken again by
-// the whole block with IEEE divisions: everything a pass writes comes out of its inputs (but x,
-// which only the first updates), so taking it twice is the same as once.
-template <class M, class Of, class At, class Next>
-DEV void down_pass(const Geo& g, int count, bool top, Of&& of, At&& at, Next&& next) {
-    if (count == 0) return;
-    const bool bad = down_pass_<M, false>(g, count, top, of, at, next);
-    if constexpr (!M::kMixed) {
-        if (__syncthreads_or(bad)) down_pass_<M, true>(g, count, top, of, at, next);
-    }
 }
 
 struct UpTile {
@@ -879,12 +887,11 @@ struct UpTile {
 
 // mg_up.comp on this block's tiles of a level: the coarse correction with omega and the
 // mirrored sweep. On level 0 (top) the tile's sums of r.z into part[tile].xy.
-template <class M, bool SLOW, class Of, class At, class Next>
-DEV bool up_pass_(const Geo& g, int count, bool top, Of&& of, At&& at, Next&& next) {
+template <class M, class Of, class At, class Next>
+DEV void up_pass(const Geo& g, int count, bool top, Of&& of, At&& at, Next&& next) {
     TileSmem& S = *reinterpret_cast<TileSmem*>(dyn_smem);
     float2* const sred = reinterpret_cast<float2*>(S.red);
     const int t = threadIdx.x;
-    bool bad = false;
     using Stage = LevelStage<M>;   // (q: the red cells' pre-smoothed values, then their coarse ones; x: the ring's coarse ones)
     auto fetch = [&](const UpTile& T, Stage& n) {
         const DevScene& d = of(T.scene);
@@ -915,8 +922,9 @@ DEV bool up_pass_(const Geo& g, int count, bool top, Of&& of, At&& at, Next&& ne
     };
     // s / D where the cell is an unknown
     auto value = [&](float2 s, const typename M::Diag& y) {
-        if (!SLOW) bad |= M::unk(y) && !M::ok(s, y);
-        return M::template quot<SLOW>(s, y);
+        float2 z = M::quot(s, y);
+        if (__builtin_expect(M::unk(y) && !M::ok(s, y), 0)) z = M::quot_ieee(s, y);
+        return z;
     };
     auto corrected = [](float2 v, float2 zc) { return make_float2(v.x + MG_OMEGA * zc.x, v.y + MG_OMEGA * zc.y); };
     auto tree = [&](const UpTile& T, const float2* prod) {
@@ -926,7 +934,7 @@ DEV bool up_pass_(const Geo& g, int count, bool top, Of&& of, At&& at, Next&& ne
     };
     auto stage = [](int turn) -> Stage& { return *reinterpret_cast<Stage*>(dyn_smem + (turn & 1) * sizeof(TileSmem::stage) / 2); };
     int k = next(0);
-    if (k >= count) return false;
+    if (k >= count) return;
     UpTile T = at(k);
     fetch(T, stage(0));
     cp_commit();
@@ -989,15 +997,6 @@ DEV bool up_pass_(const Geo& g, int count, bool top, Of&& of, At&& at, Next&& ne
             tree(cur, n.p);
         }
         if (!more) break;
-    }
-    return bad;
-}
-template <class M, class Of, class At, class Next>
-DEV void up_pass(const Geo& g, int count, bool top, Of&& of, At&& at, Next&& next) {
-    if (count == 0) return;
-    const bool bad = up_pass_<M, false>(g, count, top, of, at, next);
-    if constexpr (!M::kMixed) {
-        if (__syncthreads_or(bad)) up_pass_<M, true>(g, count, top, of, at, next);
     }
 }
 
@@ -1111,67 +1110,81 @@ DEV void apply_pass(int count, Of&& of, At&& at, Next&& next) {
 // The tail's phases, over J cells a thread at once so that their chains overlap (past the end a
 // thread repeats the last one, whose value comes out the same).
 //
-// A half-sweep over entries p0 .. p0 + cnt - 1 of a level of width w.
-template <bool SLOW, int J>
-DEV void tail_sweep(const Tail& tl, int p0, int cnt, int w, bool& bad) {
+// A quotient out of the fast form's range is taken the IEEE way after the thread has stored its others
+// (a branch before the store lengthened every phase's chain: a solve of 128 x 72 took 2 % longer). What
+// the fast form makes of it, which need not be a number, is never stored: a slot past the end of a row
+// or of a level is read too, and its zero coupling would not hide one.
+//
+// A half-sweep over entries p0 .. p0 + cnt - 1 of a level of width w: entry p's sum, and the level's cells
+// of one colour from the other's.
+DEV float2 tail_sum(const Tail& tl, int p, int s, int w) {
+    const float4 a = tl.a[p];
+    const float2 x0 = tl.x[max(s - 1, 0)], x1 = tl.x[min(s + 1, tl.T - 1)];
+    const float2 x2 = tl.x[max(s - w, 0)], x3 = tl.x[min(s + w, tl.T - 1)];
+    return sum4(tl.r[p], mul2(a.x, x0), mul2(a.y, x1), mul2(a.z, x2), mul2(a.w, x3));
+}
+// The half-sweep's form over J cells a thread: value(p, s) is entry p's sum at slot s.
+template <int J, class Value>
+DEV void tail_cells_of(const Tail& tl, int p0, int cnt, Value&& value) {
     if ((int)(threadIdx.x & ~31u) < cnt) {
         int s[J];
         float2 z[J];
+        bool ok[J], all = true;
 #pragma unroll
         for (int j = 0; j < J; j++) {
             const int p = p0 + min((int)threadIdx.x + j * NT, cnt - 1);
             s[j] = tl.slot[p];
-            const float4 a = tl.a[p];
-            const float2 x0 = tl.x[max(s[j] - 1, 0)], x1 = tl.x[min(s[j] + 1, tl.T - 1)];
-            const float2 x2 = tl.x[max(s[j] - w, 0)], x3 = tl.x[min(s[j] + w, tl.T - 1)];
-            z[j] = quot2<SLOW>(sum4(tl.r[p], mul2(a.x, x0), mul2(a.y, x1), mul2(a.z, x2), mul2(a.w, x3)), tl.dy[p], bad);
+            const float2 v = value(p, s[j]), dy = tl.dy[p];
+            z[j] = quot2(v, dy);
+            ok[j] = quot_ok<80>(v, dy.y);
+            all &= ok[j];
         }
 #pragma unroll
-        for (int j = 0; j < J; j++) tl.x[s[j]] = z[j];
+        for (int j = 0; j < J; j++)
+            if (ok[j]) tl.x[s[j]] = z[j];
+        if (__builtin_expect(!all, 0)) {   // (a cell's unknown neighbours are the other colour's)
+#pragma unroll 1
+            for (int j = 0; j < J; j++) {
+                const int p = p0 + min((int)threadIdx.x + j * NT, cnt - 1), q = tl.slot[p];
+                tl.x[q] = quot2_ieee(value(p, q), tl.dy[p]);
+            }
+        }
     }
     __syncthreads();
 }
+template <int J>
+DEV void tail_sweep(const Tail& tl, int p0, int cnt, int w) {
+    tail_cells_of<J>(tl, p0, cnt, [&](int p, int s) { return tail_sum(tl, p, s, w); });
+}
 // The black half-sweep of a way up: its neighbours are read with their coarse correction.
-template <bool SLOW, int J>
-DEV void tail_correct(const Tail& tl, const TailLevel& L, const TailLevel& C, bool& bad) {
-    const int cnt = L.n1;
-    if ((int)(threadIdx.x & ~31u) < cnt) {
-        int s[J];
-        float2 z[J];
-#pragma unroll
-        for (int j = 0; j < J; j++) {
-            const int p = L.o + L.n0 + min((int)threadIdx.x + j * NT, cnt - 1);
-            s[j] = tl.slot[p];
-            const float4 a = tl.a[p];
-            const int k = s[j] - L.o, y = qdiv(k, L.wm), x = k - y * L.w;
-            const int m = C.o + (y >> 1) * C.w + (x >> 1);
-            auto term = [&](float w, int sn, int c) {
-                const float2 xn = tl.x[min(max(sn, 0), tl.T - 1)], xc = tl.x[min(max(c, 0), tl.T - 1)];
-                return make_float2(w * (xn.x + MG_OMEGA * xc.x), w * (xn.y + MG_OMEGA * xc.y));
-            };
-            const float2 sum = sum4(tl.r[p], term(a.x, s[j] - 1, m - 1 + (x & 1)), term(a.y, s[j] + 1, m + (x & 1)),
-                                    term(a.z, s[j] - L.w, (y & 1) ? m : m - C.w), term(a.w, s[j] + L.w, (y & 1) ? m + C.w : m));
-            z[j] = quot2<SLOW>(sum, tl.dy[p], bad);
-        }
-#pragma unroll
-        for (int j = 0; j < J; j++) tl.x[s[j]] = z[j];
-    }
-    __syncthreads();
+template <int J>
+DEV void tail_correct(const Tail& tl, const TailLevel& L, const TailLevel& C) {
+    tail_cells_of<J>(tl, L.o + L.n0, L.n1, [&](int p, int s) {
+        const float4 a = tl.a[p];
+        const int k = s - L.o, y = qdiv(k, L.wm), x = k - y * L.w;
+        const int m = C.o + (y >> 1) * C.w + (x >> 1);
+        auto term = [&](float w, int sn, int c) {
+            const float2 xn = tl.x[min(max(sn, 0), tl.T - 1)], xc = tl.x[min(max(c, 0), tl.T - 1)];
+            return make_float2(w * (xn.x + MG_OMEGA * xc.x), w * (xn.y + MG_OMEGA * xc.y));
+        };
+        return sum4(tl.r[p], term(a.x, s - 1, m - 1 + (x & 1)), term(a.y, s + 1, m + (x & 1)),
+                    term(a.z, s - L.w, (y & 1) ? m : m - C.w), term(a.w, s + L.w, (y & 1) ? m + C.w : m));
+    });
 }
 // The right-hand side of entry p of a tail level, and its first half-sweep, which starts from
 // zero: the level's even unknowns (entries below odd) are r / D. The odd ones are written before
 // anything reads them.
-template <bool SLOW>
-DEV void tail_rhs(const Tail& tl, int p, int s, int odd, float2 dy, float2 r, bool on, bool& bad) {
-    const float2 x = quot2<SLOW>(r, dy, bad);
+DEV void tail_rhs(const Tail& tl, int p, int s, int odd, float2 dy, float2 r, bool on) {
+    const float2 x = quot2(r, dy);
+    const bool ok = quot_ok<80>(r, dy.y), even = on && p < odd;
     if (on) tl.r[p] = r;
-    if (on && p < odd) tl.x[s] = x;
+    if (even && ok) tl.x[s] = x;
+    if (__builtin_expect(even && !ok, 0)) tl.x[s] = quot2_ieee(r, dy);
 }
 // The residual of the level above summed over the four cells of each entry of level C (w: the
 // width above), four lanes to an entry, one per cell: a cell that is no unknown adds nothing (the
 // sum is never -0, so leaving it out or adding +0 is the same).
-template <bool SLOW>
-DEV void tail_restrict(const Tail& tl, const TailLevel& C, int w, bool& bad) {
+DEV void tail_restrict(const Tail& tl, const TailLevel& C, int w) {
     const int cnt = 4 * (C.n0 + C.n1), b = threadIdx.x & 28;
 #pragma unroll 1
     for (int t = threadIdx.x; (t & ~31) < cnt; t += NT) {
@@ -1196,7 +1209,7 @@ DEV void tail_restrict(const Tail& tl, const TailLevel& C, int w, bool& bad) {
             v.x += __shfl_sync(0xffffffffu, ex, b + k);
             v.y += __shfl_sync(0xffffffffu, ey, b + k);
         }
-        tail_rhs<SLOW>(tl, p, cs, C.o + C.n0, cdy, v, (t & 3) == 0 && t < cnt, bad);
+        tail_rhs(tl, p, cs, C.o + C.n0, cdy, v, (t & 3) == 0 && t < cnt);
     }
     __syncthreads();
 }
@@ -1211,9 +1224,7 @@ DEV void tail_restrict(const Tail& tl, const TailLevel& C, int w, bool& bad) {
 // 250 cycles. With the way up of the level above: 12.8 -> 7.3 us (32 x 18 cells, 4 levels),
 // 17.9 -> 10.2 us (48 x 27, 6 levels).
 constexpr int kTailJ = 3;   // a first tail level has at most 1500 cells, 750 of a colour
-template <bool SLOW>
-DEV bool tail_cycle(const float2* R, const Tail& tl) {
-    bool bad = false;
+DEV void tail_cycle(const float2* R, const Tail& tl) {
     const int last = tl.nl - 1;
     TailLevel L = tl.lv[0];
     {   // (every load in flight before the first is used)
@@ -1231,21 +1242,21 @@ DEV bool tail_cycle(const float2* R, const Tail& tl) {
         for (int j = 0; j < PER; j++) {
             if ((int)(threadIdx.x & ~31u) + j * NT >= cnt) break;
             const int p = min((int)threadIdx.x + j * NT, cnt - 1);
-            tail_rhs<SLOW>(tl, p, s[j], L.n0, tl.dy[p], v[j], true, bad);
+            tail_rhs(tl, p, s[j], L.n0, tl.dy[p], v[j], true);
         }
     }
     __syncthreads();
     // a level's cells of one colour are one a thread unless there are more than a block's threads
     auto sweep = [&](bool odd) {
         const int cnt = odd ? L.n1 : L.n0, p0 = odd ? L.o + L.n0 : L.o;
-        if (cnt <= NT) tail_sweep<SLOW, 1>(tl, p0, cnt, L.w, bad);
-        else tail_sweep<SLOW, kTailJ>(tl, p0, cnt, L.w, bad);
+        if (cnt <= NT) tail_sweep<1>(tl, p0, cnt, L.w);
+        else tail_sweep<kTailJ>(tl, p0, cnt, L.w);
     };
     sweep(true);
 #pragma unroll 1
     for (int l = 0; l < last; l++) {
         const TailLevel C = tl.lv[l + 1];
-        tail_restrict<SLOW>(tl, C, L.w, bad);
+        tail_restrict(tl, C, L.w);
         L = C;
         sweep(true);
     }
@@ -1256,23 +1267,14 @@ DEV bool tail_cycle(const float2* R, const Tail& tl) {
     for (int l = last - 1; l >= 0; l--) {
         const TailLevel C = L;
         L = tl.lv[l];
-        if (L.n1 <= NT) tail_correct<SLOW, 1>(tl, L, C, bad);
-        else tail_correct<SLOW, kTailJ>(tl, L, C, bad);
+        if (L.n1 <= NT) tail_correct<1>(tl, L, C);
+        else tail_correct<kTailJ>(tl, L, C);
         sweep(false);
     }
-    return bad;
-}
-// (only where an operand left the fast quotients' range, which may have left NaN in the iterates:
-// a zero coupling does not hide one)
-static __device__ __noinline__ void tail_slow(const float2* R, int T, int nf, int nl) {
-    const Tail tl = tail_at(dyn_smem + kTileBytes, reinterpret_cast<float2*>(dyn_smem), 0, T, nf, nl);
-    for (int s = threadIdx.x; s < T; s += NT) tl.x[s] = make_float2(0.0f, 0.0f);
-    __syncthreads();
-    tail_cycle<true>(R, tl);
 }
 // (Z: where the first tail level's result goes, for inspection; a batch's way up reads it)
 DEV void phase_tail(const float2* R, float2* Z, const Tail& tl) {
-    if (__syncthreads_or(tail_cycle<false>(R, tl))) tail_slow(R, tl.T, tl.nf, tl.nl);
+    tail_cycle(R, tl);
     if (Z)
         for (int s = threadIdx.x; s < tl.nf; s += NT) Z[s] = tl.x[s];
 }

@@ -62,9 +62,13 @@ DEV float quot_fast(float a, float D, float y) {
     const float e = fmaf(q0, D, -a);
     return fmaf(-e, y, q0);
 }
-DEV bool quot_ok(float a) {
-    const float v = fabsf(a);
-    return (v >= 0x1p-80f && v <= 0x1p80f) || v == 0.0f;
+// Whether both of a are zero or within [2^-E, 2^E], and y (the reciprocal of recip, of a positive D)
+// is a number: on the bits without their sign, a chain about as long as the quotient's own.
+template <int E>
+DEV bool quot_ok(float2 a, float y) {
+    constexpr uint32_t LO = (uint32_t)(127 - E) << 24, HI = (uint32_t)(127 + E) << 24;   // bits of 2^-E, 2^E, times 2
+    const uint32_t u = __float_as_uint(a.x) << 1, v = __float_as_uint(a.y) << 1, w = __float_as_uint(y) << 1;
+    return min(u - 1u, v - 1u) >= LO - 1u && max(max(u, v), w) <= HI;   // (zero less one is above all)
 }
 // the reciprocal quot_fast wants of a positive D (0 for one that is not positive)
 DEV float recip(float D) {
@@ -77,29 +81,16 @@ DEV bool coupling_ok(float w) {
     const float v = fabsf(w);
     return (v >= 0x1p-25f && v <= 0x1p25f) || v == 0.0f;
 }
-DEV bool value_ok(float a) {
-    const float v = fabsf(a);
-    return (v >= 0x1p-60f && v <= 0x1p60f) || v == 0.0f;
-}
 DEV float recip_row(float D, float4 a) {
     const float y = recip(D);
     if (!(D > 0.0f)) return y;
     return coupling_ok(a.x) && coupling_ok(a.y) && coupling_ok(a.z) && coupling_ok(a.w) ? y : __int_as_float(0x7fffffff);
 }
-// Both columns' a / D for dy = (D, recip(D)), D > 0. The fast form notes operands outside its
-// range in `bad` and the caller then runs the same code once more with SLOW, the IEEE division:
-// a division at every use, inlined or called, was most of the persistent kernels' code, which
-// then missed the instruction cache in every phase. A diagonal that is not positive leaves
-// its (zero) numerator as it is.
-template <bool SLOW>
-DEV float quot1(float a, float2 dy) {
-    if (SLOW) return dy.x > 0.0f ? divz(a, dy.x) : a;
-    return quot_fast(a, dy.x, dy.y);
-}
-template <bool SLOW>
-DEV float2 quot2(float2 a, float2 dy, bool& bad) {
-    if (!SLOW) bad |= !(quot_ok(a.x) && quot_ok(a.y) && dy.y > 0.0f);
-    return make_float2(quot1<SLOW>(a.x, dy), quot1<SLOW>(a.y, dy));
+// Both columns' a / D for dy = (D, recip(D)): the fast way, and the IEEE division. A diagonal that is
+// not positive leaves its (zero) numerator as it is.
+DEV float2 quot2(float2 a, float2 dy) { return make_float2(quot_fast(a.x, dy.x, dy.y), quot_fast(a.y, dy.x, dy.y)); }
+DEV float2 quot2_ieee(float2 a, float2 dy) {
+    return dy.x > 0.0f ? make_float2(divz(a.x, dy.x), divz(a.y, dy.x)) : a;
 }
 
 DEV unsigned long long global_ns() {
