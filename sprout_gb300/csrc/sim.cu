@@ -746,6 +746,7 @@ struct SproutSim {
     static constexpr uint32_t kPerWorker = 16384;
     static constexpr int kSettleWorkers = 16;
     static int settle_workers(uint32_t n) {
+        if (n < 2 * kPerWorker) return 1;
         cpu_set_t cpus;   // those this process may run on: threads sharing one are slower than one alone
         const int have = sched_getaffinity(0, sizeof cpus, &cpus) == 0 ? CPU_COUNT(&cpus) : 1;
         return std::max(1, std::min({have, (int)(n / kPerWorker), (int)kSettleWorkers}));
@@ -764,10 +765,25 @@ struct SproutSim {
         for (; w < workers; w++) f(w);
         for (std::thread& t : ts) t.join();
     }
-    // in[0 .. n) with ids from 0, settled, into out; their materials added to present and *th.
-    // Returns the first particle with a non-finite position, or n.
+    // in[lo .. hi) with its indexes as ids, settled, into out; their materials added to present and *th.
+    // Returns the first particle with a non-finite position (present and *th are then as they were), or hi.
+    uint32_t settle_part(const SproutParticle* in, uint32_t lo, uint32_t hi, SproutParticle* out, bool* present, bool* th) const {
+        std::copy(in + lo, in + hi, out + lo);
+        for (uint32_t k = lo; k < hi; k++) {
+            out[k].id = k;
+            if (!settle_one(out[k])) return k;
+        }
+        // (into locals: the caller's bytes, written once a particle, were waited for by the next)
+        bool mine[kMaxMaterials] = {}, any = false;
+        mark_materials(out + lo, hi - lo, mine, &any);
+        for (int m = 0; m < kMaxMaterials; m++) present[m] |= mine[m];
+        *th |= any;
+        return hi;
+    }
+    // ... of all of in[0 .. n), by as many threads as there are parts.
     uint32_t settle_all(const SproutParticle* in, uint32_t n, SproutParticle* out, bool* present, bool* th) const {
         const int workers = settle_workers(n);
+        if (workers == 1) return settle_part(in, 0, n, out, present, th);
         struct Part {
             uint32_t bad;
             bool present[kMaxMaterials], th;
@@ -776,16 +792,8 @@ struct SproutSim {
         each_worker(workers, [&](int w) {
             const uint32_t lo = (uint32_t)((uint64_t)n * w / workers), hi = (uint32_t)((uint64_t)n * (w + 1) / workers);
             Part mine{n, {}, false};   // (on the worker's own stack until it is done)
-            std::copy(in + lo, in + hi, out + lo);
-            uint32_t k = lo;
-            for (SproutParticle* const ps = out; k < hi; k++) {
-                ps[k].id = k;
-                if (!settle_one(ps[k])) {
-                    mine.bad = k;
-                    break;
-                }
-            }
-            if (k == hi) mark_materials(out + lo, hi - lo, mine.present, &mine.th);
+            const uint32_t k = settle_part(in, lo, hi, out, mine.present, &mine.th);
+            if (k < hi) mine.bad = k;
             parts[w] = mine;
         });
         uint32_t bad = n;
