@@ -653,12 +653,14 @@ struct SproutSim {
 
     // Particle::settle_spawn (params.rs:70-85) and the position range every substep leaves a
     // particle in, [2.01, size - 2.01] (particles.comp:912), so that the first gather's 3 x 3
-    // stencils stay on the grid. False for a non-finite position.
+    // stencils stay on the grid. False for a non-finite position or a material that is no row.
     int settle(SproutParticle& q, uint32_t k) const {
-        return settle_one(q) ? SPROUT_OK : fail(SPROUT_E_ARG, "particle " + std::to_string(k) + " has a non-finite position");
+        if (settle_one(q)) return SPROUT_OK;
+        const bool finite = std::isfinite(q.pos[0]) && std::isfinite(q.pos[1]);
+        return fail(SPROUT_E_ARG, "particle " + std::to_string(k) + (finite ? " has no material row of the table" : " has a non-finite position"));
     }
     bool settle_one(SproutParticle& q) const {
-        if (!std::isfinite(q.pos[0]) || !std::isfinite(q.pos[1])) return false;
+        if (!std::isfinite(q.pos[0]) || !std::isfinite(q.pos[1]) || (q.kind & 255u) > (uint32_t)kMaxMaterials) return false;
         q.pos[0] = std::min(std::max(q.pos[0], 2.01f), (float)W - 2.01f);
         q.pos[1] = std::min(std::max(q.pos[1], 2.01f), (float)H - 2.01f);
         uint32_t mat = q.kind & 255u;
@@ -766,7 +768,7 @@ struct SproutSim {
         for (std::thread& t : ts) t.join();
     }
     // in[lo .. hi) with its indexes as ids, settled, into out; their materials added to present and *th.
-    // Returns the first particle with a non-finite position (present and *th are then as they were), or hi.
+    // Returns the first particle that settle refuses (present and *th are then as they were), or hi.
     uint32_t settle_part(const SproutParticle* in, uint32_t lo, uint32_t hi, SproutParticle* out, bool* present, bool* th) const {
         std::copy(in + lo, in + hi, out + lo);
         for (uint32_t k = lo; k < hi; k++) {
