@@ -815,10 +815,10 @@ DEV void down_pass(const Geo& g, int count, bool top, Of&& of, At&& at, Next&& n
         r = f2sel(unk, r, -0.0f);
         er = f2sel(eunk, er, -0.0f);
         if (g.red) {
-            const bool odd = unk && !M::ok(r, y);
+            const bool out = unk && !M::ok(r, y);
             float2 z = M::quot(r, y);
-            if (__builtin_expect(odd, 0)) z = M::quot_ieee(r, y);
-            S.red[g.s] = M::pack_red(r, odd ? M::spoilt(y) : y);
+            if (__builtin_expect(out, 0)) z = M::quot_ieee(r, y);
+            S.red[g.s] = M::pack_red(r, out ? M::spoilt(y) : y);
             if (in) of(cur.scene).mgx[i] = f2sel(unk, z, 0.0f);
             if (g.kind == 2) S.red[g.es] = M::pack_red(er, eunk && !M::ok(er, ey) ? M::spoilt(ey) : ey);
         }
