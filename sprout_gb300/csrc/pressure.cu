@@ -1221,8 +1221,8 @@ DEV void tail_restrict(const Tail& tl, const TailLevel& C, int w) {
 //
 // It is a chain of ~24 block-wide phases of a few cells each, bound by each phase's latency:
 // two dependent shared-memory reads, eight dependent adds and multiplies and a fast quotient, about
-// 250 cycles. With the way up of the level above: 12.8 -> 7.3 us (32 x 18 cells, 4 levels),
-// 17.9 -> 10.2 us (48 x 27, 6 levels).
+// 250 cycles. With the way up of the level above: 12.8 -> 6.4 us (32 x 18 cells, 4 levels),
+// 17.9 -> 8.0 us (48 x 27, 6 levels).
 constexpr int kTailJ = 3;   // a first tail level has at most 1500 cells, 750 of a colour
 DEV void tail_cycle(const float2* R, const Tail& tl) {
     const int last = tl.nl - 1;
@@ -1279,7 +1279,7 @@ DEV void phase_tail(const float2* R, float2* Z, const Tail& tl) {
         for (int s = threadIdx.x; s < tl.nf; s += NT) Z[s] = tl.x[s];
 }
 
-// The active-tile lists of levels 0 .. tail - 1 of scene d (one block), from ptile.
+// The active-tile list of level l (below the tail) of scene d, from ptile (one block).
 DEV void build_plist(const DevScene& d, int l) {
     const Lv L = lev(d.lv, l);
     compact_flags(d.ptile + L.toff, tiles_x(L) * tiles_y(L), d.plist + L.toff, d.pcount + l);
